@@ -258,7 +258,7 @@ __device__ void merge_prep(G g, int a, int mid, int b, int n, double* Z, const d
     }
     dm = group_max(g, dm, red);
     zm = group_max(g, zm, red);
-    const double tol = 8.0 * kEps * fmax(dm, zm);
+    const double tol = 8.0 * kEps * fmax(dm, rho * zm);   // both are energies: independent of the matrix's scale
     g.sync();
     if (t == 0) {
         int K = 0, ndf = 0, nrot = 0, jlam = -1;
