@@ -31,6 +31,7 @@ enum : int {
     NRG_DEV_SMEM = 2,            // a block did not fit the configured shared memory
     NRG_DEV_SECULAR = 4,         // a secular root did not bracket
     NRG_DEV_NONFINITE = 8,       // NaN/Inf met in an input block
+    NRG_DEV_TIMEOUT = 16,        // a bounded wait between blocks expired
 };
 
 // --------------------------------------------------------------------------------------
@@ -53,6 +54,12 @@ __host__ __device__ inline long long syev_ws_doubles(long long n) {
 }
 __host__ __device__ inline long long syev_ws_ints(long long n) { return 12 * n + 64; }
 
+// offset of D | E | tau (n doubles each) and the divide-and-conquer vectors in it
+__host__ __device__ inline long long syev_vec_off(long long n) {
+    const long long sq = n * n;
+    return 2 * sq + (sq > 64 * n ? sq : 64 * n);
+}
+
 // launch helpers implemented in the .cu files (return NRG status)
-int launch_syev(const SyevSector* d_secs, int nsec, int max_n, double* eigbuf, double* evals,
-                double* wsd, int* wsi, int* d_status, cudaStream_t st);
+int launch_tri_small(const SyevSector* d_secs, int nsec, double* eigbuf, double* wsd, int* d_status, cudaStream_t st);
+int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* wsi, int* d_status, cudaStream_t st);

@@ -2,8 +2,8 @@
 // iteration (the dsyev('V','U') call of diagonalization.F90:267, one call per sector),
 // one thread block per sector.  Used for blocks of order <= 128 (large blocks go through
 // the multi-kernel pipeline of eig_large.cu, which reuses the pieces below):
-//   1. Householder tridiagonalisation of the lower triangle (H = Q T Q^T), in shared
-//      memory for orders <= 128, reflectors kept in the block's own storage;
+//   1. Householder tridiagonalisation (H = Q T Q^T) by a launch of its own with the block in
+//      registers (eig_tri.cu), reflectors kept in the block's own storage;
 //   2. divide and conquer on T (Cuppen tearing down to 1x1 leaves, deflation of small
 //      z components and of close pole pairs by Givens rotations, secular roots by a
 //      safeguarded rational iteration in pole-shifted coordinates, Gu-Eisenstat
@@ -20,64 +20,7 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kNB = 32;           // reflectors per back-transform panel
-constexpr int kSmemTri = 128;     // orders tridiagonalised in shared memory
 constexpr int kDcCap = 128;       // orders whose divide and conquer vectors live in shared memory
-
-// Householder tridiagonalisation of the n x n block A (leading dim lda, full storage kept
-// symmetric); reflector k is stored below the subdiagonal of column k with an implicit 1.
-__device__ void tridiagonalise(double* A, int lda, int n, double* Dd, double* Ee, double* TAU,
-                               double* vs, double* ps, double* red) {
-    const int tid = threadIdx.x, T = blockDim.x;
-    for (int k = 0; k < n - 1; ++k) {
-        const int m = n - k - 1;
-        double* col = A + (size_t)k * lda;
-        const double alpha = col[k + 1];
-        double part = 0.0;
-        for (int i = k + 2 + tid; i < n; i += T) part += col[i] * col[i];
-        const double xn2 = block_sum(part, red);
-        if (xn2 == 0.0) {
-            if (tid == 0) { Ee[k] = alpha; TAU[k] = 0.0; }
-            continue;
-        }
-        const double beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-        const double tt = (beta - alpha) / beta;
-        const double scal = 1.0 / (alpha - beta);
-        for (int i = tid; i < m; i += T) {
-            double vi = 1.0;
-            if (i > 0) { vi = col[k + 1 + i] * scal; col[k + 1 + i] = vi; }
-            vs[i] = vi;
-        }
-        if (tid == 0) { Ee[k] = beta; TAU[k] = tt; }
-        __syncthreads();
-        double pv_part = 0.0;
-        for (int i = tid; i < m; i += T) {
-            const double* Ai = A + (size_t)(k + 1 + i) + (size_t)(k + 1) * lda;
-            double s0 = 0.0, s1 = 0.0;
-            int j = 0;
-            for (; j + 1 < m; j += 2) {
-                s0 = fma(Ai[(size_t)j * lda], vs[j], s0);
-                s1 = fma(Ai[(size_t)(j + 1) * lda], vs[j + 1], s1);
-            }
-            if (j < m) s0 = fma(Ai[(size_t)j * lda], vs[j], s0);
-            const double pi = tt * (s0 + s1);
-            ps[i] = pi;
-            pv_part += pi * vs[i];
-        }
-        const double pv = block_sum(pv_part, red);
-        const double h = -0.5 * tt * pv;
-        for (int i = tid; i < m; i += T) ps[i] += h * vs[i];
-        __syncthreads();
-        for (int j = 0; j < m; ++j) {
-            const double vj = vs[j], wj = ps[j];
-            double* Aj = A + (size_t)(k + 1) + (size_t)(k + 1 + j) * lda;
-            for (int i = tid; i < m; i += T) Aj[i] -= vs[i] * wj + ps[i] * vj;
-        }
-        __syncthreads();
-    }
-    for (int k = tid; k < n; k += T) Dd[k] = A[(size_t)k + (size_t)k * lda];
-    if (tid == 0) Ee[n - 1] = 0.0;
-    __syncthreads();
-}
 
 // back-transformation Z <- Q Z with Q = H_0 ... H_{n-2} (reflectors in A), kNB at a time
 __device__ void back_transform(const double* A, int n, const double* TAU, double* Z, double* Vb,
@@ -153,7 +96,7 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
                                                     double* __restrict__ eigbuf,
                                                     double* __restrict__ evals,
                                                     double* __restrict__ wsd, int* __restrict__ wsi,
-                                                    int* status, int smem_tri) {
+                                                    int* status) {
     extern __shared__ double sm[];
     const SyevSector sec = secs[blockIdx.x];
     const int n = sec.n;
@@ -181,8 +124,7 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
     double* Z = W;
     double* U = W + sq;
     double* Qt = W + 2 * sq;
-    const long long qt = sq > 64LL * n ? sq : 64LL * n;
-    double* vec = W + 2 * sq + qt;
+    double* vec = W + syev_vec_off(n);
     double* Dd = vec;
     double* Ee = vec + n;
     double* TAU = vec + 2 * n;
@@ -191,22 +133,8 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
 
     double* red = sm;
     double* gsm = sm + 32;
-    double* vs = sm + 32 + nrg::kCtaGemmSmem;
-    const int vlen = n > kNB * kNB ? n : kNB * kNB;
-    double* ps = vs + vlen;
-    double* dcs = vs + 2 * vlen + kNB * kNB;          // D and the merge vectors (orders <= kDcCap)
-    double* As = dcs + kDcSmemDoubles * kDcCap;
-
-    // ---- 1. tridiagonalisation ----
-    if (smem_tri && n <= kSmemTri) {
-        for (long long e = tid; e < sq; e += T) As[e] = A[e];
-        __syncthreads();
-        tridiagonalise(As, n, n, Dd, Ee, TAU, vs, ps, red);
-        for (long long e = tid; e < sq; e += T) A[e] = As[e];
-        __syncthreads();
-    } else {
-        tridiagonalise(A, n, n, Dd, Ee, TAU, vs, ps, red);
-    }
+    double* vs = sm + 32 + nrg::kCtaGemmSmem;          // T and the Gram matrix of a back-transformation panel
+    double* dcs = vs + 2 * kNB * kNB;                   // D and the merge vectors (orders <= kDcCap)
 
     // ---- 2. divide and conquer on (Dd, Ee) -> eigenvalues in Dm, vectors in Z ----
     double* Dm = Dd;
@@ -252,19 +180,12 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
 
 }  // namespace
 
-int launch_syev(const SyevSector* d_secs, int nsec, int max_n, double* eigbuf, double* evals,
-                double* wsd, int* wsi, int* d_status, cudaStream_t st) {
+int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* wsi, int* d_status, cudaStream_t st) {
     if (nsec == 0) return NRG_OK;
-    const size_t vlen = (size_t)(max_n > kNB * kNB ? max_n : kNB * kNB);
-    const int smem_tri = max_n <= kSmemTri ? 1 : 0;
-    size_t smem = sizeof(double) * (32 + nrg::kCtaGemmSmem + 2 * vlen + kNB * kNB + kDcSmemDoubles * kDcCap +
-                                    (smem_tri ? (size_t)max_n * max_n : 0));
-    if (smem > 227 * 1024) {
-        nrg_set_error_message("sector of order %d exceeds the shared-memory plan", max_n);
-        return NRG_ERR_TOO_LARGE;
-    }
+    NRG_TRY(launch_tri_small(d_secs, nsec, eigbuf, wsd, d_status, st));
+    const size_t smem = sizeof(double) * (32 + nrg::kCtaGemmSmem + 2 * kNB * kNB + kDcSmemDoubles * kDcCap);
     if (smem > 48 * 1024) NRG_TRY(nrg::raise_smem_limit((const void*)k_syev, smem));
-    k_syev<<<nsec, kThreads, smem, st>>>(d_secs, eigbuf, evals, wsd, wsi, d_status, smem_tri);
+    k_syev<<<nsec, kThreads, smem, st>>>(d_secs, eigbuf, evals, wsd, wsi, d_status);
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
 }

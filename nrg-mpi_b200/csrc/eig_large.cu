@@ -1,6 +1,8 @@
 // FP64 eigensolver for the large symmetry sectors of one iteration (order > 128), spread
 // over the whole GPU instead of one block per sector.  All large sectors advance together:
-//   1. blocked Householder tridiagonalisation (panels of 32 columns, the dlatrd scheme):
+//   1. Householder tridiagonalisation: orders up to 512 with the matrix on chip
+//      (eig_tri.cu), larger ones by panels until the trailing block fits there.  The panel
+//      scheme (32 columns, dlatrd):
 //      per column one block per sector updates the column with the pending panel
 //      reflectors and forms the Householder vector, then a many-block kernel computes the
 //      symmetric matrix-vector product with the trailing matrix (column dot products,
@@ -35,7 +37,8 @@ constexpr int kTriCL16Min = 1 << 30;   // order from which a launch takes 16-blo
 
 struct LSec {
     long long a_off, e_off, w_off, i_off;
-    int n, pad;
+    int n;
+    int stop;   // columns the panel kernel reduces: n - 1, or fewer when the rest goes on chip
 };
 
 // workspace per sector: Z, U, Qt (n x n each), the panel V | W (n x 2 NB), y, the D&C
@@ -314,7 +317,7 @@ __global__ void __launch_bounds__(TT, 1) k_tri_cluster(const LSec* __restrict__ 
     // CL is even, so every own column's offset (rank + CL m) n has the parity of rank n
     const int par = (int)(((reinterpret_cast<uintptr_t>(A) >> 3) + (uintptr_t)rank * n) & 1);
 
-    for (int p = 0; p < n - 1; p += NB) {
+    for (int p = 0; p < sec.stop; p += NB) {
         const int last = min(p + NB - 1, n - 2);
         const int jn = last - p + 1;
         // rows p..last of the own columns: the panel's columns read them as rows (the
@@ -602,8 +605,10 @@ __global__ void __launch_bounds__(TT, 1) k_tri_cluster(const LSec* __restrict__ 
             __syncthreads();
         }
     }
-    if ((n - 1) % CL == rank && tid == 0) L.D[n - 1] = A[(size_t)(n - 1) + (size_t)(n - 1) * n];
-    if (rank == 0 && tid == 0) L.E[n - 1] = 0.0;
+    if (sec.stop == n - 1) {
+        if ((n - 1) % CL == rank && tid == 0) L.D[n - 1] = A[(size_t)(n - 1) + (size_t)(n - 1) * n];
+        if (rank == 0 && tid == 0) L.E[n - 1] = 0.0;
+    }
     cluster.sync();   // no block leaves while another may still write its shared memory
 }
 
@@ -1466,6 +1471,22 @@ static int tri_csym_cl(nrg_context* ctx, const LSec* dsec, int ns, int maxn, dou
     return NRG_OK;
 }
 
+static int tri_forced() {
+    static const int forced = [] {
+        const char* e = getenv("NRG_TRI_CLUSTER");
+        if (!e || !*e) return -1;
+        const int v = atoi(e);
+        return (v == 0 || v == 4 || v == 8 || v == 16) ? v : -1;
+    }();
+    return forced;
+}
+static bool tri_sym() {
+    static const bool sym = [] {
+        const char* e = getenv("NRG_TRI_SYM");
+        return e && e[0] == '1';
+    }();
+    return sym;
+}
 // Cluster size of the one-launch tridiagonalisation: 8 blocks per sector (16 for the
 // largest size class alone halves its per-block product but costs as much in the wider
 // exchanges: no net gain measured); a size that cannot be placed falls back to the next
@@ -1476,16 +1497,8 @@ static int tri_csym_cl(nrg_context* ctx, const LSec* dsec, int ns, int maxn, dou
 // so the full-column kernel is the default.
 static int tri_cluster(nrg_context* ctx, const LSec* dsec, int ns, int maxn, double* d_V, double* wsd,
                        int* wsi, bool* done) {
-    static const int forced = [] {
-        const char* e = getenv("NRG_TRI_CLUSTER");
-        if (!e || !*e) return -1;
-        const int v = atoi(e);
-        return (v == 0 || v == 4 || v == 8 || v == 16) ? v : -1;
-    }();
-    static const bool sym = [] {
-        const char* e = getenv("NRG_TRI_SYM");
-        return e && e[0] == '1';
-    }();
+    const int forced = tri_forced();
+    const bool sym = tri_sym();
     // launches whose largest sector reaches this order take 16-block clusters: their
     // column product (the trailing matrix streamed from L2) outweighs the wider exchanges
     static const int cl16_min = [] {
@@ -1536,7 +1549,7 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         secs[s].a_off = in[s].a_off;
         secs[s].e_off = in[s].e_off;
         secs[s].n = in[s].n;
-        secs[s].pad = 0;
+        secs[s].stop = in[s].n - 1;
         secs[s].w_off = wd;
         secs[s].i_off = wi;
         wd += lws_doubles(in[s].n);
@@ -1552,6 +1565,14 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
     NRG_TRY(bsec.ensure(sizeof(LSec) * ns));
     NRG_TRY(bwd.ensure(sizeof(double) * (size_t)wd));
     NRG_TRY(bwi.ensure(sizeof(int) * (size_t)wi));
+    // Sectors that fit on chip are reduced there (tri_resident).  A larger one goes
+    // through the panel kernel until its trailing block fits: nbig of them, the first ones
+    // (the list is sorted by decreasing order).
+    const bool resident = tri_forced() < 0 && !tri_sym();
+    const int res_max = tri_resident_max();
+    int nbig = 0;
+    while (nbig < ns && (!resident || secs[nbig].n > res_max)) ++nbig;
+    for (int s = 0; resident && s < nbig; ++s) secs[s].stop = (secs[s].n - res_max + NB - 1) / NB * NB;
     NRG_TRY(h2d_async(ctx, bsec.p, secs.data(), sizeof(LSec) * ns));
     const LSec* dsec = bsec.as<LSec>();
     double* wsd = bwd.as<double>();
@@ -1580,7 +1601,18 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         NRG_CUDA_TRY(cudaEventCreate(&te[1]));
         NRG_CUDA_TRY(cudaEventRecord(te[0], st));
     }
-    NRG_TRY(tri_cluster(ctx, dsec, ns, maxn, d_V, wsd, wsi, &clustered));
+    if (nbig > 0) NRG_TRY(tri_cluster(ctx, dsec, nbig, maxn, d_V, wsd, wsi, &clustered));
+    else clustered = true;
+    if (resident) {
+        std::vector<TriItem> items;
+        for (int x = clustered ? 0 : nbig; x < ns; ++x) {
+            const int n = secs[x].n, c = x < nbig ? secs[x].stop : 0;   // columns done by the panels
+            double* vec = wsd + secs[x].w_off + 3LL * n * n + 2LL * NB * n + n;
+            items.push_back(TriItem{d_V + secs[x].a_off + c + (long long)c * n, vec + c, vec + n + c, vec + 2 * n + c,
+                                    n - c, n});
+        }
+        NRG_TRY(tri_resident(ctx, items, ctx->scratch.b[slot_base == 24 ? 46 : 47]));
+    }
     if (ctx->profiling) {
         NRG_CUDA_TRY(cudaEventRecord(te[1], st));
         if (clustered) {
@@ -1600,18 +1632,18 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         for (int j = 0; j < NB; ++j) {
             const int k = p + j;
             if (k > maxn - 2) break;
-            k_tri_col<<<ns, TPB, 0, st>>>(dsec, k, d_V, wsd, wsi);
+            k_tri_col<<<nbig, TPB, 0, st>>>(dsec, k, d_V, wsd, wsi);
             int nblk = 0;
-            for (int s = 0; s < ns; ++s)
+            for (int s = 0; s < nbig; ++s)
                 if (k <= secs[s].n - 2) nblk += (secs[s].n - k - 1 + CB - 1) / CB;
-            k_tri_symv<<<nblk, TPB, symv_smem, st>>>(dsec, ns, k, d_V, wsd, wsi);
+            k_tri_symv<<<nblk, TPB, symv_smem, st>>>(dsec, nbig, k, d_V, wsd, wsi);
             ctx->launches += 2;
         }
-        k_tri_finish<<<ns, TPB, 0, st>>>(dsec, p, d_V, wsd, wsi);
+        k_tri_finish<<<nbig, TPB, 0, st>>>(dsec, p, d_V, wsd, wsi);
         ctx->launches++;
         NRG_CUDA_TRY(cudaGetLastError());
         std::vector<GemmProblem> probs;
-        for (int s = 0; s < ns; ++s) {
+        for (int s = 0; s < nbig; ++s) {
             const int n = secs[s].n;
             const int c = std::min(p + NB - 1, n - 2);
             if (c < p) continue;
@@ -1630,7 +1662,7 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         NRG_TRY(launch_ggemm(ctx, probs, gslot));
     }
     if (!clustered) {
-        k_tri_end<<<ns, 32, 0, st>>>(dsec, d_V, wsd, wsi);
+        k_tri_end<<<nbig, 32, 0, st>>>(dsec, d_V, wsd, wsi);
         ctx->launches++;
     }
 

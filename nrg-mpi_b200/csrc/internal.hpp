@@ -279,6 +279,17 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& secs, double* d_
                cudaEvent_t evals_ready = nullptr);
 constexpr int kLargeSector = 128;
 
+// tridiagonalisation with the matrix resident on chip (eig_tri.cu): D, E, tau and the
+// reflectors (below the subdiagonal of A) of every item, on ctx->stream; orders 2 ..
+// tri_resident_max()
+struct TriItem {
+    double* A;             // full symmetric storage, leading dimension lda
+    double *D, *E, *TAU;
+    int n, lda;
+};
+int tri_resident_max();
+int tri_resident(nrg_context* ctx, const std::vector<TriItem>& items, DevBuf& tasks);
+
 // ---- kernels (kernels.cu) ------------------------------------------------------------
 int run_assemble(nrg_context* ctx, int iteration, const Sectors& S, const SyevSector* d_secs,
                  const long long* d_colPrefix, const int* d_secStart, int nsec, long long ncols,

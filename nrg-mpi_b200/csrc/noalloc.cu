@@ -142,7 +142,7 @@ extern "C" int nrg_block_eigh_noalloc(const double* H, int32_t n, double* eigenv
     NRG_CUDA_TRY(cudaMemcpyAsync(d_sec, &sec, sizeof(sec), cudaMemcpyHostToDevice, st));
     if (eigenvectors != H)
         NRG_CUDA_TRY(cudaMemcpyAsync(eigenvectors, H, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st));
-    NRG_TRY(launch_syev(d_sec, 1, n, eigenvectors, eigenvalues, d_ws, d_ints, d_status, st));
+    NRG_TRY(launch_syev(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_ints, d_status, st));
     int flags = 0;
     NRG_CUDA_TRY(cudaMemcpyAsync(&flags, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     NRG_CUDA_TRY(cudaStreamSynchronize(st));

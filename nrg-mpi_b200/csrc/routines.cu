@@ -315,7 +315,7 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
     std::vector<long long> colPrefix(nsec);
     std::vector<int> secStart(nsec);
     long long wsd = 0, wsi = 0, cols = 0;
-    int max_n = 1, nlarge = 0;
+    int nlarge = 0;
     std::vector<SyevSector> large;
     for (int x = 0; x < nsec; ++x) {
         const int s = order[x];
@@ -334,7 +334,6 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
             q.i_off = wsi;
             wsd += syev_ws_doubles(q.n);
             wsi += syev_ws_ints(q.n);
-            max_n = std::max(max_n, q.n);
         }
         colPrefix[x] = cols;
         cols += q.n;
@@ -403,9 +402,9 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
     }
     if (fork_small) NRG_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
     if (nsec > nlarge && rl == NRG_OK) {
-        rl = launch_syev(bsec.as<SyevSector>() + nlarge, nsec - nlarge, max_n, d_V, d_E, bwd.as<double>(),
+        rl = launch_syev(bsec.as<SyevSector>() + nlarge, nsec - nlarge, d_V, d_E, bwd.as<double>(),
                          bwi.as<int>(), ctx->d_status.as<int>(), fork_small ? ctx->aux : ctx->stream);
-        ctx->launches++;
+        ctx->launches += 2;
     }
     if (fork_small) NRG_CUDA_TRY(cudaEventRecord(ctx->ev_join, ctx->aux));
     const bool has_g2 = fork_large && !g2.empty();
