@@ -4,100 +4,152 @@
 // the multi-kernel pipeline of eig_large.cu, which reuses the pieces below):
 //   1. Householder tridiagonalisation (H = Q T Q^T) by a launch of its own with the block in
 //      registers (eig_tri.cu), reflectors kept in the block's own storage;
-//   2. divide and conquer on T (Cuppen tearing down to 1x1 leaves, deflation of small
-//      z components and of close pole pairs by Givens rotations, secular roots by a
+//   2. divide and conquer on T (eig_dc.cuh: Cuppen tearing down to 1x1 leaves, deflation of
+//      small z components and of close pole pairs by Givens rotations, secular roots by a
 //      safeguarded rational iteration in pole-shifted coordinates, Gu-Eisenstat
-//      recomputation of z for orthogonal eigenvectors); merges of up to 32 rows run one
-//      per warp, larger merges use the whole block and an in-block tiled GEMM;
-//   3. back-transformation V = Q Z with 32 reflectors at a time (compact WY form,
-//      two in-block GEMMs per panel).
+//      recomputation of z for orthogonal eigenvectors);
+//   3. back-transformation V = Q Z with 32 reflectors at a time (compact WY form), the
+//      columns of Z in registers.
 // Eigenvalues come out ascending with their eigenvectors in the same column order, as
 // dsyev returns them.
-#include "eig_common.cuh"
+#include "eig_dc.cuh"
 #include "internal.hpp"
 
 namespace {
 
-constexpr int kThreads = 512;
+constexpr int kThreads = kLeafThreads;
 constexpr int kNB = 32;           // reflectors per back-transform panel
-constexpr int kDcCap = 128;       // orders whose divide and conquer vectors live in shared memory
 
-// back-transformation Z <- Q Z with Q = H_0 ... H_{n-2} (reflectors in A), kNB at a time
-__device__ void back_transform(const double* A, int n, const double* TAU, double* Z, double* Vb,
-                               double* Qt, double* Ts, double* Gs, double* gsm) {
-    const int tid = threadIdx.x, T = blockDim.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int nr = n - 1;
-    for (int jb = ((nr - 1) / kNB) * kNB; jb >= 0; jb -= kNB) {
-        const int b = min(kNB, nr - jb);
-        const int r0 = jb + 1, mr = n - r0;
-        for (long long e = tid; e < (long long)mr * b; e += T) {
-            const int i = (int)(e % mr), c = (int)(e / mr);
-            const int k = jb + c, row = r0 + i;
-            double v = 0.0;
-            if (row == k + 1) v = 1.0;
-            else if (row > k + 1) v = A[(size_t)row + (size_t)k * n];
-            Vb[e] = v;
-        }
-        __syncthreads();
-        for (int e = tid; e < b * b; e += T) {
-            const int p = e % b, q = e / b;
-            double s = 0.0;
-            if (p < q) {
-                const double* vp = Vb + (size_t)p * mr;
-                const double* vq = Vb + (size_t)q * mr;
-                for (int i = 0; i < mr; ++i) s = fma(vp[i], vq[i], s);
+// Back-transformation V = Q Z with Q = H_0 ... H_{n-2}, 32 reflectors at a time (compact
+// WY form), n <= 128.  Every warp keeps eight columns of Z in registers, transposed, as the
+// accumulators of its MMA tiles; the three products of a panel, W^T = Z^T V, W2^T = W^T T^T
+// and Z^T -= W2^T V^T, hand their accumulators on as A operands.  An accumulator's columns
+// 2 q, 2 q + 1 of a lane are taken as the k index q of two MMAs (the order of a sum's terms
+// is free), so no product's result moves between lanes: only V and T come from shared memory
+// and the warps never wait for one another.  Bound by the FP64 MMA rate of one SM (2 n^3
+// operations, 17 us at n = 128).
+constexpr int kMaxN = 128;                       // order
+constexpr int kLdV = kMaxN + 4;                  // Vs[k * kLdV + row]; = 4 mod 16
+constexpr int kLdT = kNB + 4;                    // Ts[q][k * kLdT + n] = T_q(n, k); Gs alike
+constexpr int kPanels = kMaxN / kNB;
+constexpr size_t kBtSmem = sizeof(double) * (kMaxN * kLdV + 2 * kPanels * kNB * kLdT);
+static_assert(kBtSmem <= kLeafSmem, "the back-transformation reuses the divide and conquer's shared memory");
+
+// row (or reflector) of position i of an 8-wide tile, so that a lane's accumulator columns
+// 2 q, 2 q + 1 are rows q and q + 4
+__device__ __forceinline__ int tile_pos(int i) { return (i >> 1) + 4 * (i & 1); }
+
+__device__ void back_transform(double* A, int n, const double* TAU, const double* Z, double* sm) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q4 = lane & 3;
+    double* Vs = sm;
+    double* Ts = Vs + kMaxN * kLdV;
+    double* Gs = Ts + kPanels * kNB * kLdT;
+    const int nr = n - 1, np = (nr + kNB - 1) / kNB, nt = (n + 7) / 8;
+    // the reflectors of every panel (zeros above, beyond n and beyond the last one)
+    for (int k = warp; k < np * kNB; k += kThreads / 32)
+        for (int row = lane; row < 8 * nt; row += 32)
+            Vs[k * kLdV + row] = k >= nr || row >= n || row <= k ? 0.0 : (row == k + 1 ? 1.0 : A[(size_t)row + (size_t)k * n]);
+    __syncthreads();
+    // Gram matrices G_q = V_q^T V_q, four warps per panel, one row of 8 x 8 tiles each
+    {
+        const int q = warp >> 2, r = warp & 3;
+        if (q < np) {
+            double acc[4][2];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[c][0] = acc[c][1] = 0.0;
+            for (int i0 = kNB * q; i0 < 8 * nt; i0 += 4) {
+                const double a = Vs[(kNB * q + 8 * r + g) * kLdV + i0 + q4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (c >= r) nrg::cta_dmma(acc[c][0], acc[c][1], a, Vs[(kNB * q + 8 * c + g) * kLdV + i0 + q4]);
             }
-            Gs[p + q * kNB] = s;
-            Ts[p + q * kNB] = 0.0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (c >= r)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) Gs[q * kNB * kLdT + (8 * r + g) * kLdT + 8 * c + 2 * q4 + h] = acc[c][h];
         }
-        __syncthreads();
-        if (warp == 0) {
-            for (int c = 0; c < b; ++c) {
-                const double tc = TAU[jb + c];
-                double acc = 0.0;
-                if (lane < c)
-                    for (int q = lane; q < c; ++q) acc += Ts[lane + q * kNB] * (-tc * Gs[q + c * kNB]);
-                __syncwarp();
-                if (lane < c) Ts[lane + c * kNB] = acc;
-                if (lane == 0) Ts[c + c * kNB] = tc;
-                __syncwarp();
+    }
+    __syncthreads();
+    // T_q (dlarft, forward, columnwise): one warp per panel, row `lane` of T in registers
+    if (warp < np) {
+        const double* G = Gs + warp * kNB * kLdT;
+        double* T = Ts + warp * kNB * kLdT;
+        double row[kNB];
+#pragma unroll
+        for (int c = 0; c < kNB; ++c) {
+            const int k = kNB * warp + c;
+            const double tc = k < nr ? TAU[k] : 0.0;
+            double s[2] = {0.0, 0.0};
+#pragma unroll
+            for (int q = 0; q < c; ++q) s[q & 1] = fma(row[q], G[q * kLdT + c], s[q & 1]);
+            row[c] = lane == c ? tc : (lane < c ? -tc * (s[0] + s[1]) : 0.0);
+            T[c * kLdT + lane] = row[c];
+        }
+    }
+    __syncthreads();
+    // this warp's columns
+    const int col = 8 * warp + g;
+    double z[kMaxN / 8][2];
+#pragma unroll
+    for (int t = 0; t < kMaxN / 8; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = 8 * t + q4 + 4 * h;
+            z[t][h] = t < nt && row < n && col < n ? Z[(size_t)row + (size_t)col * n] : 0.0;
+        }
+    if (8 * warp < n) {
+        for (int q = np - 1; q >= 0; --q) {
+            const double* V = Vs + kNB * q * kLdV;
+            const double* T = Ts + q * kNB * kLdT;
+            double w[4][2], w2[4][2];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) w[c][0] = w[c][1] = w2[c][0] = w2[c][1] = 0.0;
+#pragma unroll
+            for (int t = 0; t < kMaxN / 8; ++t)
+                if (t >= 4 * q && t < nt) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            nrg::cta_dmma(w[c][0], w[c][1], z[t][h], V[(8 * c + tile_pos(g)) * kLdV + 8 * t + q4 + 4 * h]);
+                }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int d = 0; d < 4; ++d)
+                        if (d <= c) nrg::cta_dmma(w2[d][0], w2[d][1], w[c][h], T[(8 * c + q4 + 4 * h) * kLdT + 8 * d + tile_pos(g)]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) w2[c][h] = -w2[c][h];
+#pragma unroll
+            for (int t = 0; t < kMaxN / 8; ++t)
+                if (t >= 4 * q && t < nt) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            nrg::cta_dmma(z[t][0], z[t][1], w2[c][h], V[(8 * c + q4 + 4 * h) * kLdV + 8 * t + tile_pos(g)]);
+                }
+        }
+#pragma unroll
+        for (int t = 0; t < kMaxN / 8; ++t)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int row = 8 * t + q4 + 4 * h;
+                if (t < nt && row < n && col < n) A[(size_t)row + (size_t)col * n] = z[t][h];
             }
-        }
-        __syncthreads();
-        double* Wm = Qt;
-        double* W2 = Qt + (size_t)kNB * n;
-        {
-            auto fa = [=](int i, int k) -> double { return Vb[(size_t)k + (size_t)i * mr]; };
-            auto fb = [=](int k, int j) -> double { return Z[(size_t)(r0 + k) + (size_t)j * n]; };
-            auto fc = [=](int i, int j) -> double& { return Wm[(size_t)i + (size_t)j * b]; };
-            nrg::cta_gemm(b, n, mr, 1.0, 0.0, fa, fb, fc, gsm);
-        }
-        __syncthreads();
-        for (long long e = tid; e < (long long)b * n; e += T) {
-            const int p = (int)(e % b);
-            const long long j = e / b;
-            double s = 0.0;
-            for (int q = p; q < b; ++q) s = fma(Ts[p + q * kNB], Wm[(size_t)q + (size_t)j * b], s);
-            W2[e] = s;
-        }
-        __syncthreads();
-        {
-            auto fa = [=](int i, int k) -> double { return Vb[(size_t)i + (size_t)k * mr]; };
-            auto fb = [=](int k, int j) -> double { return W2[(size_t)k + (size_t)j * b]; };
-            auto fc = [=](int i, int j) -> double& { return Z[(size_t)(r0 + i) + (size_t)j * n]; };
-            nrg::cta_gemm(mr, n, b, -1.0, 1.0, fa, fb, fc, gsm);
-        }
-        __syncthreads();
     }
 }
 
 __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict__ secs,
                                                     double* __restrict__ eigbuf,
                                                     double* __restrict__ evals,
-                                                    double* __restrict__ wsd, int* __restrict__ wsi,
-                                                    int* status) {
-    extern __shared__ double sm[];
+                                                    double* __restrict__ wsd, int* status) {
+    extern __shared__ __align__(16) double sm[];
     const SyevSector sec = secs[blockIdx.x];
     const int n = sec.n;
     const int tid = threadIdx.x, T = blockDim.x;
@@ -120,62 +172,19 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
         return;
     }
     double* W = wsd + sec.w_off;
-    const long long sq = (long long)n * n;
     double* Z = W;
-    double* U = W + sq;
-    double* Qt = W + 2 * sq;
     double* vec = W + syev_vec_off(n);
     double* Dd = vec;
     double* Ee = vec + n;
     double* TAU = vec + 2 * n;
-    int* I = wsi + sec.i_off;
-    Scratch S = scratch_at(vec, I, n);
 
-    double* red = sm;
-    double* gsm = sm + 32;
-    double* vs = sm + 32 + nrg::kCtaGemmSmem;          // T and the Gram matrix of a back-transformation panel
-    double* dcs = vs + 2 * kNB * kNB;                   // D and the merge vectors (orders <= kDcCap)
-
-    // ---- 2. divide and conquer on (Dd, Ee) -> eigenvalues in Dm, vectors in Z ----
-    double* Dm = Dd;
-    Scratch Sm = S;
-    if (n <= kDcCap) {
-        Dm = dcs;
-        Sm = scratch_smem(dcs, kDcCap);
-    }
-    for (long long e = tid; e < sq; e += T) Z[e] = 0.0;
-    __syncthreads();
-    for (int i = tid; i < n; i += T) {
-        Z[(size_t)i + (size_t)i * n] = 1.0;
-        double dv = Dd[i];
-        if (i > 0) dv -= fabs(Ee[i - 1]);
-        if (i < n - 1) dv -= fabs(Ee[i]);
-        Dm[i] = dv;
-    }
-    __syncthreads();
-    const int warp = tid >> 5, lane = tid & 31, nwarps = T >> 5;
-    for (int s = 1; s < n; s *= 2) {
-        if (2 * s <= 32) {
-            WarpG wg{lane};
-            int mi = 0;
-            for (int a = 0; a + s < n; a += 2 * s, ++mi) {
-                if (mi % nwarps != warp) continue;
-                dc_merge(wg, a, a + s, min(a + 2 * s, n), n, Z, Dm, Ee, Sm, U, Qt, red, gsm, status);
-            }
-            __syncthreads();
-        } else {
-            BlockG bg;
-            for (int a = 0; a + s < n; a += 2 * s)
-                dc_merge(bg, a, a + s, min(a + 2 * s, n), n, Z, Dm, Ee, Sm, U, Qt, red, gsm, status);
-        }
-    }
+    // ---- 2. divide and conquer on (Dd, Ee) -> eigenvalues in Dd, vectors in Z ----
+    dc_leaf(0, n, n, Dd, Ee, Z, sm, status);
     __syncthreads();
 
-    // ---- 3. back-transformation ----
-    back_transform(A, n, TAU, Z, U, Qt, vs, vs + kNB * kNB, gsm);
-
-    for (int i = tid; i < n; i += T) ev[i] = Dm[i];
-    for (long long e = tid; e < sq; e += T) A[e] = Z[e];
+    // ---- 3. back-transformation, straight to the output ----
+    back_transform(A, n, TAU, Z, sm);
+    for (int i = tid; i < n; i += T) ev[i] = Dd[i];
 }
 
 }  // namespace
@@ -183,9 +192,8 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
 int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* wsi, int* d_status, cudaStream_t st) {
     if (nsec == 0) return NRG_OK;
     NRG_TRY(launch_tri_small(d_secs, nsec, eigbuf, wsd, d_status, st));
-    const size_t smem = sizeof(double) * (32 + nrg::kCtaGemmSmem + 2 * kNB * kNB + kDcSmemDoubles * kDcCap);
-    if (smem > 48 * 1024) NRG_TRY(nrg::raise_smem_limit((const void*)k_syev, smem));
-    k_syev<<<nsec, kThreads, smem, st>>>(d_secs, eigbuf, evals, wsd, wsi, d_status);
+    NRG_TRY(nrg::raise_smem_limit((const void*)k_syev, kLeafSmem));
+    k_syev<<<nsec, kThreads, kLeafSmem, st>>>(d_secs, eigbuf, evals, wsd, d_status);
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
 }

@@ -1,30 +1,22 @@
-// Device building blocks of the FP64 symmetric eigensolver shared by the one-block-per-
-// sector kernel (eig.cu) and the multi-kernel pipeline for large sectors (eig_large.cu):
-// reductions, the divide-and-conquer merge in phases, and the secular-equation solver.
+// Device building blocks of the FP64 symmetric eigensolver: reductions, and the phases of
+// the divide-and-conquer merges that are spread over the whole device (eig_large.cu), with
+// the secular-equation solver.  (Merges of up to 128 rows run in one block: eig_dc.cuh.)
 #pragma once
 #include "common.cuh"
 #include "cta_gemm.cuh"
 
 #include <math.h>
-#include <type_traits>
 
 namespace {
 
 constexpr double kEps = 1.1102230246251565e-16;
 
-// a whole block or one warp
+// the threads of a whole block
 struct BlockG {
     __device__ int rank() const { return threadIdx.x; }
     __device__ int size() const { return blockDim.x; }
     __device__ void sync() const { __syncthreads(); }
 };
-struct WarpG {
-    int lane;
-    __device__ int rank() const { return lane; }
-    __device__ int size() const { return 32; }
-    __device__ void sync() const { __syncwarp(); }
-};
-
 __device__ double block_sum(double v, double* red) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -48,10 +40,6 @@ __device__ double block_max(double v, double* red) {
     return s;
 }
 __device__ double group_max(BlockG, double v, double* red) { return block_max(v, red); }
-__device__ double group_max(WarpG, double v, double*) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 
 // scratch arrays of one sector, each of length n, indexed by absolute row
 struct Scratch {
@@ -67,22 +55,6 @@ __device__ Scratch scratch_at(double* vec, int* I, int n) {
     S.rc = vec + 11 * n; S.rs = vec + 12 * n;
     S.perm = I; S.nd = I + n; S.df = I + 2 * n; S.org = I + 3 * n; S.pos = I + 4 * n;
     S.ra = I + 5 * n; S.rb = I + 6 * n; S.mk = I + 7 * n; S.mr = I + 8 * n; S.mf = I + 9 * n;
-    return S;
-}
-
-// The same vectors for a range of at most cap rows in shared memory, indexed from the
-// start of the range: cap doubles for D, then 10 cap doubles and 10 cap ints (16 cap
-// doubles in all, from dsm).  The merges' serial and iterative parts (deflation scan,
-// secular roots, ranks) then wait on shared memory instead of L2.
-constexpr int kDcSmemDoubles = 16;
-__device__ Scratch scratch_smem(double* dsm, int cap) {
-    Scratch S;
-    double* v = dsm + cap;
-    int* I = reinterpret_cast<int*>(dsm + 11 * cap);
-    S.z = v; S.ds = v + cap; S.zs = v + 2 * cap; S.dd = v + 3 * cap; S.zz = v + 4 * cap;
-    S.tau = v + 5 * cap; S.zh = v + 6 * cap; S.vals = v + 7 * cap; S.rc = v + 8 * cap; S.rs = v + 9 * cap;
-    S.perm = I; S.nd = I + cap; S.df = I + 2 * cap; S.org = I + 3 * cap; S.pos = I + 4 * cap;
-    S.ra = I + 5 * cap; S.rb = I + 6 * cap; S.mk = I + 7 * cap; S.mr = I + 8 * cap; S.mf = I + 9 * cap;
     return S;
 }
 
@@ -117,8 +89,6 @@ struct GroupLanes {
     }
 };
 using WarpLanes = GroupLanes<32>;
-// lanes per item inside the one-block merges
-constexpr int kMergeLanes = 4;
 
 // Root j of 1 + rho * sum_i zz_i^2 / (dd_i - lambda) = 0 (rho > 0, dd ascending, zz != 0),
 // returned as lambda = dd[org] + tau with org the pole nearer to the root, so that every
@@ -417,51 +387,6 @@ __device__ void merge_copyback(int t, int T, int a, int b, int n, double* Z, dou
         Z[(size_t)(a + i) + (size_t)(a + c) * n] = Qt[(size_t)(a + i) + (size_t)(a + c) * n];
     }
     for (int e = t; e < nn; e += T) D[a + S.pos[a + e]] = S.vals[a + e];
-}
-
-// the whole merge inside one group
-template <class G>
-__device__ void dc_merge(G g, int a, int mid, int b, int n, double* Z, double* D,
-                         const double* E, Scratch S, double* U, double* Qt, double* red,
-                         double* gsm, int* status) {
-    const int t = g.rank(), T = g.size();
-    const int nn = b - a;
-    const GroupLanes<kMergeLanes> gl{(int)(threadIdx.x & 31)};
-    merge_prep(g, a, mid, b, n, Z, D, E, S, red);
-    g.sync();
-    merge_roots(t / kMergeLanes, T / kMergeLanes, a, mid, E, S, status, gl);
-    g.sync();
-    merge_zhat(t / kMergeLanes, T / kMergeLanes, a, mid, E, S, gl);
-    g.sync();
-    merge_ucols(t / kMergeLanes, T / kMergeLanes, a, n, S, U, gl);
-    merge_vals(t, T, a, b, S);
-    g.sync();
-    merge_rank(t, T, a, b, S);
-    g.sync();
-    const int K = S.mk[a];
-    if constexpr (std::is_same<G, BlockG>::value) {
-        const int* perm = S.perm + a;
-        const int* nd = S.nd + a;
-        const int* pos = S.pos + a;
-        auto fa = [=](int i, int k) -> double { return Z[(size_t)(a + i) + (size_t)(a + perm[nd[k]]) * n]; };
-        auto fb = [=](int k, int j) -> double { return U[(size_t)(a + k) + (size_t)(a + j) * n]; };
-        auto fc = [=](int i, int j) -> double& { return Qt[(size_t)(a + i) + (size_t)(a + pos[j]) * n]; };
-        if (K > 0) nrg::cta_gemm(nn, K, K, 1.0, 0.0, fa, fb, fc, gsm);
-    } else {
-        for (int i = t; i < nn; i += T) {
-            for (int j = 0; j < K; ++j) {
-                double s = 0.0;
-                for (int q = 0; q < K; ++q)
-                    s += Z[(size_t)(a + i) + (size_t)(a + S.perm[a + S.nd[a + q]]) * n] *
-                         U[(size_t)(a + q) + (size_t)(a + j) * n];
-                Qt[(size_t)(a + i) + (size_t)(a + S.pos[a + j]) * n] = s;
-            }
-        }
-    }
-    merge_deflated(t, T, a, b, n, Z, Qt, S);
-    g.sync();
-    merge_copyback(t, T, a, b, n, Z, D, Qt, S);
-    g.sync();
 }
 
 }  // namespace

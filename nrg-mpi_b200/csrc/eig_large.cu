@@ -13,7 +13,7 @@
 //      final order) with the eigenvector update Z(:, kept) * U as a grouped GEMM;
 //   3. back-transformation in panels of 64 reflectors: Gram matrix and V^T Z as grouped
 //      GEMMs, the triangular factor T in one block, then Z -= (V T)(V^T Z).
-#include "eig_common.cuh"
+#include "eig_dc.cuh"
 #include "internal.hpp"
 
 #include <cooperative_groups.h>
@@ -29,7 +29,7 @@ namespace {
 
 constexpr int NB = 32;        // tridiagonalisation panel
 constexpr int NBB = 64;       // back-transformation panel
-constexpr int DC_LOW = 128;   // merges of up to this many rows run inside one block
+constexpr int DC_LOW = kDcLeafRows;   // merges of up to this many rows run inside one block
 constexpr int TPB = 256;
 constexpr int CB = 32;        // columns per block in the symmetric matrix-vector product
 constexpr int kTriCL = 8;     // blocks per cluster of the one-launch tridiagonalisation
@@ -961,9 +961,9 @@ __global__ void k_tri_end(const LSec* __restrict__ secs, double* eigbuf, double*
 // ---------------------------------------------------------------------------------
 // leaves of the divide and conquer: one block per aligned range of DC_LOW rows of a
 // sector runs every merge inside that range (all merges up to DC_LOW rows stay inside)
-__global__ void __launch_bounds__(512) k_dc_low(const LSec* __restrict__ secs, int nsec, double* eigbuf,
+__global__ void __launch_bounds__(kLeafThreads) k_dc_low(const LSec* __restrict__ secs, int nsec, double* eigbuf,
                                                 double* wsd, int* wsi, int* status) {
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];
     int bid = blockIdx.x, sidx = 0;
     for (; sidx < nsec; ++sidx) {
         const int nc = (secs[sidx].n + DC_LOW - 1) / DC_LOW;
@@ -972,50 +972,8 @@ __global__ void __launch_bounds__(512) k_dc_low(const LSec* __restrict__ secs, i
     }
     if (sidx >= nsec) return;
     LView L = lview(secs[sidx], eigbuf, wsd, wsi);
-    const int n = L.n, tid = threadIdx.x, T = blockDim.x;
-    const int c0 = bid * DC_LOW, c1 = min(c0 + DC_LOW, n), nl = c1 - c0;
-    double* red = sm;
-    double* gsm = sm + 32;
-    // D of the range and the merge vectors in shared memory; the merges work in indices
-    // local to the range (Z, U, Qt through pointers to the range's diagonal block)
-    double* Dl = gsm + nrg::kCtaGemmSmem;
-    const Scratch Sl = scratch_smem(Dl, DC_LOW);
-    double* Zl = L.Z + c0 + (size_t)c0 * n;
-    double* Ul = L.U + c0 + (size_t)c0 * n;
-    double* Ql = L.Qt + c0 + (size_t)c0 * n;
-    const double* El = L.E + c0;
-    // columns c0 .. c1-1 of Z start as the identity
-    const long long ne = (long long)n * (c1 - c0);
-    for (long long e = tid; e < ne; e += T) {
-        const long long col = c0 + e / n, row = e % n;
-        L.Z[row + col * n] = (row == col) ? 1.0 : 0.0;
-    }
-    // rank-one tearing at every boundary: each leaf is 1 x 1
-    for (int i = c0 + tid; i < c1; i += T) {
-        double dv = L.D[i];
-        if (i > 0) dv -= fabs(L.E[i - 1]);
-        if (i < n - 1) dv -= fabs(L.E[i]);
-        Dl[i - c0] = dv;
-    }
-    __syncthreads();
-    const int warp = tid >> 5, lane = tid & 31, nwarps = T >> 5;
-    for (int s = 1; 2 * s <= DC_LOW && s < nl; s *= 2) {
-        if (2 * s <= 32) {
-            WarpG wg{lane};
-            int mi = 0;
-            for (int a = 0; a + s < nl; a += 2 * s, ++mi) {
-                if (mi % nwarps != warp) continue;
-                dc_merge(wg, a, a + s, min(a + 2 * s, nl), n, Zl, Dl, El, Sl, Ul, Ql, red, gsm, status);
-            }
-            __syncthreads();
-        } else {
-            BlockG bg;
-            for (int a = 0; a + s < nl; a += 2 * s)
-                dc_merge(bg, a, a + s, min(a + 2 * s, nl), n, Zl, Dl, El, Sl, Ul, Ql, red, gsm, status);
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < nl; i += T) L.D[c0 + i] = Dl[i];
+    const int c0 = bid * DC_LOW;
+    dc_leaf(c0, min(DC_LOW, L.n - c0), L.n, L.D, L.E, L.Z, sm, status);
 }
 
 struct Merge {
@@ -1668,10 +1626,10 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
 
     // ---- 2. divide and conquer ----
     {
-        const size_t smem = sizeof(double) * (32 + nrg::kCtaGemmSmem + kDcSmemDoubles * DC_LOW);
+        NRG_TRY(raise_smem_limit((const void*)k_dc_low, kLeafSmem));
         int nchunk = 0;
         for (int x = 0; x < ns; ++x) nchunk += (secs[x].n + DC_LOW - 1) / DC_LOW;
-        k_dc_low<<<nchunk, 512, smem, st>>>(dsec, ns, d_V, wsd, wsi, ctx->d_status.as<int>());
+        k_dc_low<<<nchunk, kLeafThreads, kLeafSmem, st>>>(dsec, ns, d_V, wsd, wsi, ctx->d_status.as<int>());
         ctx->launches++;
         NRG_CUDA_TRY(cudaGetLastError());
     }
