@@ -31,6 +31,7 @@
 // column for 6.5..7; order 128 0.20 ms for 0.9 (the one-block code it replaces), 512 1.2 ms
 // for 3.3.  Whole runs: N_keep = 250 37.5 ms for 53, N_keep = 2048 with the FDM spectrum
 // 453 ms for 567, eight models side by side 146 ms for 218.
+#include "cta_gemm.cuh"
 #include "internal.hpp"
 
 #include <algorithm>
@@ -69,8 +70,12 @@ struct Plan {
     static constexpr int kMax = NR < CL * kCols ? NR : CL * kCols;   // largest order
     // shared memory, in doubles: the exchange buffers (two of y | a per row and of the
     // blocks' parts of u.y), two barriers, v | w and x by row, the column sums by row
-    // group, row k + 1 of the own columns, the warps' parts of u.y, scalars
-    static constexpr int kBuf = 0, kUY = kBuf + (CL > 1 ? 4 * NR : 0), kBar = kUY + 2 * CL;
+    // group, row k + 1 of the own columns, the warps' parts of u.y, scalars.  Row i of an
+    // exchange buffer is at (i % CL) kSrc + i / CL: what one block sends is contiguous, and
+    // with kSrc odd consecutive rows still lie on different banks.
+    static constexpr int kSrc = kCols | 1, kEx = CL * kSrc;
+    static constexpr int kBuf = 0, kUY = kBuf + (CL > 1 ? 4 * kEx : 0), kBar = kUY + 2 * CL;
+    __host__ __device__ static constexpr int at(int i) { return (i % CL) * kSrc + i / CL; }
     static constexpr int kVW = kBar + 2, kX = kVW + 2 * NR, kPart = kX + NR, kRow = kPart + G * kCols;
     static constexpr int kP = kRow + kCols, kScal = kP + kTriWarps, kDoubles = kScal + 8;
     static constexpr size_t kBytes = sizeof(double) * kDoubles;
@@ -166,12 +171,11 @@ template <class P>
 __device__ __forceinline__ void tri_init(const TriTask& t, double* sm) {
     const int tid = threadIdx.x, n = t.n;
     // step 0 reads y = 0 and column 0, and the scalars of no reflector
+    if constexpr (P::CL > 1)
+        for (int i = tid; i < n; i += kTriThreads)
+            reinterpret_cast<double2*>(sm + P::kBuf)[P::at(i)] = make_double2(0.0, t.A[i]);
     for (int i = tid; i < P::NR; i += kTriThreads) {
-        if constexpr (P::CL > 1) {
-            double2* buf = reinterpret_cast<double2*>(sm + P::kBuf);
-            buf[i] = make_double2(0.0, i < n ? t.A[i] : 0.0);
-            buf[P::NR + i] = make_double2(0.0, 0.0);
-        } else if (i < P::kCols) {
+        if constexpr (P::CL == 1) if (i < P::kCols) {
             sm[P::kPart + i] = 0.0;
             sm[P::kRow + i] = i < n ? t.A[i] : 0.0;
         }
@@ -200,6 +204,34 @@ __device__ __forceinline__ void tri_load(const TriTask& t, double* sm, double (&
 // scalars of the current reflector, from the ninth warp (after kScal)
 enum { kTau = 0, kH = 1, kAlpha = 2, kDiag = 3, kScale = 4 };
 
+// beta, tau, u(k+1) and the factor of the normalised reflector, from the sum of squares
+// below alpha; un: the factor that u takes itself
+struct Reflector {
+    double beta, h, tau, scal, un;
+};
+__device__ __forceinline__ Reflector reflector(double ss, double al) {
+    Reflector r{al, 0.0, 0.0, 0.0, 1.0};
+    if (ss == 0.0) return r;
+    const double q = fma(al, al, ss);
+    // the root and the quotients from rsqrt and reciprocals: sqrt and a general division
+    // take four to six times as long
+    if (q > 1e-150 && q < 1e150) {
+        const double s = rsqrt(q), b = q * s;
+        r.beta = -copysign(fma(0.5 * s, fma(-b, b, q), b), al);
+        r.h = al - r.beta;
+        r.tau = 1.0 / (-r.beta * r.h);
+        r.scal = 1.0 / r.h;
+    } else {
+        // far from one the squares and cubes of u would leave the range: normalise
+        r.beta = -copysign(sqrt(q), al);
+        r.un = 1.0 / (al - r.beta);
+        r.tau = (r.beta - al) / r.beta;
+        r.h = 1.0;
+        r.scal = r.un;
+    }
+    return r;
+}
+
 // the norm of x, beta, tau and u(k+1) of column k, and the stores of the reflector
 template <class P>
 __device__ __forceinline__ void tri_norm(const TriTask& t, double* sm, int k) {
@@ -214,40 +246,20 @@ __device__ __forceinline__ void tri_norm(const TriTask& t, double* sm, int k) {
         s1 = fma(x1, x1, s1);
     }
     if (i < n) s0 = fma(xs[i], xs[i], s0);
-    const double ss = bfly(s0 + s1), al = sc[kAlpha];
-    const double q = fma(al, al, ss);
-    double beta = al, hn = 0.0, tau = 0.0, scal = 0.0, un = 1.0;
-    if (ss != 0.0) {
-        // the root and the quotients from rsqrt and reciprocals: sqrt and a general
-        // division take four to six times as long
-        if (q > 1e-150 && q < 1e150) {
-            const double r = rsqrt(q), b = q * r;
-            beta = -copysign(fma(0.5 * r, fma(-b, b, q), b), al);
-            hn = al - beta;
-            tau = 1.0 / (-beta * hn);
-            scal = 1.0 / hn;
-        } else {
-            // far from one the squares and cubes of u would leave the range: normalise
-            beta = -copysign(sqrt(q), al);
-            un = 1.0 / (al - beta);
-            tau = (beta - al) / beta;
-            hn = 1.0;
-            scal = un;
-        }
-    }
+    const Reflector f = reflector(bfly(s0 + s1), sc[kAlpha]);
     if (lane == 0) {
-        sc[kTau] = tau;
-        sc[kH] = hn;
-        sc[kScale] = un;
+        sc[kTau] = f.tau;
+        sc[kH] = f.h;
+        sc[kScale] = f.un;
     }
     if ((k + 1) % P::CL == t.rank) {   // a block that is in the loop as long as this column
         double* ref = t.A + (size_t)k * t.lda;
         for (int r = ((k + 2) & ~31) + lane; r < n; r += 32)
-            if (r >= k + 2) ref[r] = xs[r] * scal;
+            if (r >= k + 2) ref[r] = xs[r] * f.scal;
         if (lane == 0) {
             t.D[k] = sc[kDiag];
-            t.E[k] = beta;
-            t.TAU[k] = hn * hn * tau;   // (beta - alpha) / beta
+            t.E[k] = f.beta;
+            t.TAU[k] = f.h * f.h * f.tau;   // (beta - alpha) / beta
         }
     }
 }
@@ -350,7 +362,7 @@ __device__ __forceinline__ void tri_steps(const TriTask& t, double* sm, double (
             const double tau = sc[kTau], h = sc[kH];
             auto ya_of = [&](int i) {
                 if constexpr (CL > 1) {
-                    return reinterpret_cast<const double2*>(sm + P::kBuf)[b * NR + i];
+                    return reinterpret_cast<const double2*>(sm + P::kBuf)[b * P::kEx + P::at(i)];
                 } else {
                     double y = part[i];
 #pragma unroll
@@ -460,14 +472,16 @@ __device__ __forceinline__ void tri_steps(const TriTask& t, double* sm, double (
             if (k < n - 2) {
                 const double h = sc[kH];
                 const unsigned bar = bar0 + 8 * (b ^ 1);
-                for (int e = tid; e < cnt * CL; e += kTriRows) {
-                    const int m = e / CL, r = e % CL, j = rank + CL * m;
-                    if (j >= rk) {
+                // a warp sends 32 columns to one block at a time
+                constexpr int kParts = (P::kCols + 31) / 32;
+                for (int e = warp; e < CL * kParts; e += kTriWarps) {
+                    const int r = e % CL, m = 32 * (e / CL) + lane;
+                    if (m < cnt && rank + CL * m >= rk) {
                         double y = part[m];
 #pragma unroll
                         for (int g = 1; g < G; ++g) y += part[g * P::kCols + m];
                         const double av = rowv[m];
-                        send16(map_rank(buf0 + 16 * ((b ^ 1) * NR + j), base + r), fma(h, av, y), av,
+                        send16(map_rank(buf0 + 16 * ((b ^ 1) * P::kEx + rank * P::kSrc + m), base + r), fma(h, av, y), av,
                                map_rank(bar, base + r));
                     }
                 }
@@ -535,6 +549,469 @@ __global__ void __launch_bounds__(kTriThreads, 1) k_tri_res(const TriTask* __res
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
+// ---------------------------------------------------------------------------------
+// larger orders: the matrix streamed from L2 until the trailing block fits on chip
+// ---------------------------------------------------------------------------------
+// The same step with the tile in global memory (L2): column j in block j % CL, columns
+// full.  Up to NBS rank-2 updates are kept back as vectors u_q, w_q, replicated in every
+// block's shared memory, so that a step only reads the matrix; then one pass applies them
+// (FP64 MMA, inner length 2 NBS).  The sums that arrive are those of the matrix as stored:
+//   a = A(k, :) - sum_q (u_q(k) w_q + w_q(k) u_q),   y = A x - sum_q (u_q (w_q.x) + w_q (u_q.x)),
+// with w_q.x and u_q.x from a run of rows per block, sent beside the column sums: still one
+// message per step.  Bound by the L2 stream of a block (8 m^2 / CL bytes per step, m the
+// trailing order, at 37 of the 44..48 bytes per cycle that eight warps reach) and, below m
+// of about 600, by the chain of the step.  Order 1225: 9.8 ms to order 512 and 1.1 ms on
+// chip, against 17.2 ms of the cluster kernel with panels of 32 columns and two cluster
+// barriers per column that it replaced (8 blocks; with 16 that one was no faster).
+constexpr int kStreamSlots = 7;   // kept updates at most (NBS), fewer where they do not fit
+
+struct StreamTask {
+    double *A, *D, *E, *TAU;
+    int n, stop, rank, keep;   // stop: columns to reduce; keep: updates kept back
+};
+
+struct StreamLayout {
+    int ld, nr, cols, keep;
+    __host__ __device__ StreamLayout(int n, int CL, int keep_) {
+        ld = ((n + 1 + 15) & ~15) + 4;            // = 4 mod 16: conflict-free MMA operands
+        cols = ((n + CL - 1) / CL) | 1;           // row i of an exchange buffer: (i % CL) cols + i / CL
+        nr = CL * cols;
+        keep = keep_;
+    }
+    __host__ __device__ int u() const { return 0; }
+    __host__ __device__ int w() const { return (keep + 1) * ld; }
+    __host__ __device__ int buf() const { return 2 * (keep + 1) * ld; }
+    __host__ __device__ int dots(int) const { return buf() + 4 * nr; }
+    __host__ __device__ int uy(int CL) const { return dots(CL) + 4 * keep * CL; }
+    __host__ __device__ int bar(int CL) const { return uy(CL) + 2 * CL; }
+    __host__ __device__ int tsum(int CL) const { return bar(CL) + 2; }
+    __host__ __device__ int part(int CL) const { return tsum(CL) + 8 * kStreamSlots; }
+    __host__ __device__ int row(int CL) const { return part(CL) + cols; }
+    __host__ __device__ int p(int CL) const { return (row(CL) + cols + 1) & ~1; }
+    __host__ __device__ int scal(int CL) const { return p(CL) + kTriWarps; }
+    __host__ __device__ int doubles(int CL) const { return scal(CL) + 8; }
+};
+
+// the sums over the warp of four values: lane l ends with the total of value (l >> 3) & 3
+__device__ __forceinline__ double sum4(const double (&a)[4], int lane) {
+    double k = quad(a, lane);
+    k += __shfl_xor_sync(kAll, k, 4);
+    k += __shfl_xor_sync(kAll, k, 2);
+    return k + __shfl_xor_sync(kAll, k, 1);
+}
+
+// the ninth warp: norm of the new column, reflector, the block's sums of u.y and of the kept
+// updates' products
+template <int CL>
+__device__ __forceinline__ void stream_norm_steps(const StreamTask& t, double* sm, unsigned to0) {
+    const int n = t.n, rank = t.rank, keep = t.keep;
+    const StreamLayout lay(n, CL, keep);
+    const int lane = threadIdx.x & 31;
+    double* U = sm + lay.u();
+    double *tsum = sm + lay.tsum(CL), *pw = sm + lay.p(CL), *sc = sm + lay.scal(CL);
+    const unsigned bar0 = smem_addr(sm + lay.bar(CL)), uy0 = smem_addr(sm + lay.uy(CL)), dots0 = smem_addr(sm + lay.dots(CL));
+    const int ld = lay.ld;
+    const int par = (int)(((reinterpret_cast<uintptr_t>(t.A) >> 3) + (uintptr_t)rank * n) & 1);
+    int np = 0;                            // kept updates (complete pairs)
+    for (int k = 0; k <= t.stop; ++k) {
+        const int b = k & 1;
+        const bool fin = k == t.stop;      // only completes the last update and applies what is kept
+        const int full = np + (k > 0);     // pairs once this step has formed w
+        const bool apply = fin || full == keep;
+        const int next = apply ? 0 : full;
+        const int nw = full * ld + par;    // the new column
+        step_sync();
+        if (fin) break;
+        // the norm of the new column, beta, u(k+1) and tau; the reflector's stores
+        const double* xs = U + nw;
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        int i = k + 2 + lane;
+        for (; i + 96 < n; i += 128) {
+            s0 = fma(xs[i], xs[i], s0);
+            s1 = fma(xs[i + 32], xs[i + 32], s1);
+            s2 = fma(xs[i + 64], xs[i + 64], s2);
+            s3 = fma(xs[i + 96], xs[i + 96], s3);
+        }
+        for (; i < n; i += 32) s0 = fma(xs[i], xs[i], s0);
+        const Reflector r = reflector(bfly((s0 + s1) + (s2 + s3)), sc[kAlpha]);
+        if (lane == 0) {
+            sc[kTau] = r.tau;
+            sc[kH] = r.h;
+            sc[kScale] = r.un;
+        }
+        if ((k + 1) % CL == rank) {
+            double* ref = t.A + (size_t)k * n;
+            for (int e = k + 2 + lane; e < n; e += 32) ref[e] = xs[e] * r.scal;
+            if (lane == 0) {
+                t.D[k] = sc[kDiag];
+                t.E[k] = r.beta;
+                t.TAU[k] = r.h * r.h * r.tau;   // (beta - alpha) / beta
+            }
+        }
+        step_sync();
+        if (sc[kScale] != 1.0) step_sync();
+        const unsigned bar = bar0 + 8 * (b ^ 1);
+        if (lane < CL) {
+            double s = 0.0;
+#pragma unroll
+            for (int r = 0; r < kTriWarps; r += 2) s += pw[r] + pw[r + 1];
+            send8(map_rank(uy0 + 8 * ((b ^ 1) * CL + rank), to0 + lane), s, map_rank(bar, to0 + lane));
+        }
+        for (int e = lane; e < next * CL; e += 32) {
+            const int q = e / CL, r = e % CL;
+            send16(map_rank(dots0 + 16 * (((b ^ 1) * keep + q) * CL + rank), to0 + r), tsum[8 * q], tsum[8 * q + 1],
+                   map_rank(bar, to0 + r));
+        }
+        np = next;
+    }
+}
+
+template <int CL>
+__device__ __forceinline__ void stream_steps(const StreamTask& t, double* sm, unsigned to0, int* status) {
+    constexpr int NBS = kStreamSlots;
+    const int n = t.n, rank = t.rank, keep = t.keep;
+    const StreamLayout lay(n, CL, keep);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double *U = sm + lay.u(), *W = sm + lay.w();
+    double* tsum = sm + lay.tsum(CL);      // (w_q.x, u_q.x) of the kept updates
+    double* part = sm + lay.part(CL);
+    double* rowv = sm + lay.row(CL);
+    double* pw = sm + lay.p(CL);
+    double* sc = sm + lay.scal(CL);
+    const unsigned bar0 = smem_addr(sm + lay.bar(CL)), buf0 = smem_addr(sm + lay.buf());
+    const int cnt = (n - rank + CL - 1) / CL, ld = lay.ld;
+    // CL is even, so every own column's offset (rank + CL m) n has the parity of rank n; with
+    // vectors stored from index par on, rows pair up on 16-byte boundaries in A and in them
+    const int par = (int)(((reinterpret_cast<uintptr_t>(t.A) >> 3) + (uintptr_t)rank * n) & 1);
+    auto first_own = [&](int i0) { return (i0 - rank + CL - 1) / CL; };
+    auto ex = [&](int i) { return (int)((unsigned)i % CL) * lay.cols + (int)((unsigned)i / CL); };
+    int np = 0;                            // kept updates (complete pairs), u_q and w_q in slot q
+    bool late = false;
+    for (int k = 0; k <= t.stop; ++k) {
+        const int b = k & 1;
+        const bool fin = k == t.stop;      // only completes the last update and applies what is kept
+        const int full = np + (k > 0);     // pairs once this step has formed w
+        const bool apply = fin || full == keep;
+        const int next = apply ? 0 : full;
+        const int cur = np * ld + par, nw = full * ld + par;   // u of the last reflector, the new column
+        if (k > 0 && !late) {
+            late = !__all_sync(kAll, bar_wait(bar0 + 8 * b, ((k - 1) >> 1) & 1));
+            if (late && lane == 0) atomicOr(status, NRG_DEV_TIMEOUT);
+        }
+        // step k + 1 brings the columns from k + 1 on, and from every block its parts of
+        // u.y and of the kept updates' products
+        if (tid == 0 && !fin && k < t.stop)
+            bar_expect(bar0 + 8 * (b ^ 1), 16u * (unsigned)(n - 1 - k) + (8u + 16u * (unsigned)next) * CL);
+        if (np > 0) {
+            // totals over the blocks and what a kept update adds at row k: one warp each
+            if (warp < np) {
+                const double2* in = reinterpret_cast<const double2*>(sm + lay.dots(CL)) + (b * keep + warp) * CL;
+                double2 e = lane < CL ? in[lane] : make_double2(0.0, 0.0);
+                const double u = U[warp * ld + par + k], w = W[warp * ld + par + k];
+                e.x = bfly(e.x);
+                e.y = bfly(e.y);
+                if (lane == 0) {
+                    double2* o = reinterpret_cast<double2*>(tsum + 8 * warp);
+                    o[0] = e;
+                    o[1] = make_double2(u, w);
+                    o[2] = make_double2(fma(u, e.x, w * e.y), 2.0 * u * w);
+                    o[3].x = 2.0 * e.x * e.y;
+                }
+            }
+            asm volatile("bar.sync 2, %0;" ::"n"(kTriRows) : "memory");
+        }
+        // ---- 1. w of the last reflector and column k ----
+        const double tau = sc[kTau], h = sc[kH];
+        const double2* in = reinterpret_cast<const double2*>(sm + lay.buf()) + b * lay.nr;
+        double uk[NBS], wk[NBS], t1[NBS], t2[NBS];
+        double2 yk = in[ex(k)];
+        double s = 0.0;
+        {
+            const double2* uy = reinterpret_cast<const double2*>(sm + lay.uy(CL) + b * CL);
+#pragma unroll
+            for (int r = 0; r < CL / 2; ++r) s += uy[r].x + uy[r].y;
+        }
+#pragma unroll
+        for (int q = 0; q < NBS; ++q) {
+            uk[q] = wk[q] = t1[q] = t2[q] = 0.0;
+            if (q < np) {
+                const double2* o = reinterpret_cast<const double2*>(tsum + 8 * q);
+                const double2 e0 = o[0], e1 = o[1], e2 = o[2];
+                t1[q] = e0.x;
+                t2[q] = e0.y;
+                uk[q] = e1.x;
+                wk[q] = e1.y;
+                yk.x -= e2.x;
+                yk.y -= e2.y;
+                s -= o[3].x;
+            }
+        }
+        yk.x = fma(h, yk.y, yk.x);
+        s = fma(h, fma(-h, yk.y, 2.0 * yk.x), s);
+        const double cf = -0.5 * tau * (tau * s);
+        const double wpiv = fma(cf, h, tau * yk.x);
+        if (tid == 0) sc[kDiag] = fma(-2.0 * wpiv, h, yk.y);
+        for (int i = k + 1 + tid; i < n; i += kTriRows) {
+            double2 ya = in[ex(i)];
+#pragma unroll
+            for (int q = 0; q < NBS; ++q)
+                if (q < np) {
+                    const double uq = U[q * ld + par + i], wq = W[q * ld + par + i];
+                    ya.y = fma(-uk[q], wq, fma(-wk[q], uq, ya.y));
+                    ya.x = fma(-uq, t1[q], fma(-wq, t2[q], ya.x));
+                }
+            ya.x = fma(h, ya.y, ya.x);
+            const double u = k > 0 ? U[cur + i] : 0.0;
+            const double w = fma(cf, u, tau * ya.x);
+            if (k > 0) W[cur + i] = w;
+            if (!fin) {
+                const double x = fma(-w, h, fma(-u, wpiv, ya.y));
+                if (i == k + 1) sc[kAlpha] = x;
+                U[nw + i] = i == k + 1 ? 0.0 : x;
+            }
+        }
+        if (tid == 0) {
+            if (fin) {
+                // the last reflector's entries at row k, which stays in the trailing block
+                U[cur + k] = h;
+                W[cur + k] = wpiv;
+            } else {
+                U[nw + k] = 0.0;       // a product that starts one row early to pair the rows
+            }
+        }
+        step_sync();
+        // ---- 2. products with the new column; every warp keeps its own columns, warp + 8 i of
+        // the block's ----
+        const double* xs = U + nw;
+        const int r0 = fin ? k : k + 1, mR = first_own(r0);
+        const int mw = mR + ((warp - mR) & (kTriWarps - 1));           // the warp's first live column
+        if (apply && full > 0) {
+            // the kept updates go into the matrix on the way: 8 columns x 64 rows at a time as
+            // MMA accumulators, the next rows' entries loaded meanwhile; rows and columns
+            // beyond the end repeat the last one and are not stored
+            const int g = lane >> 2, q4 = lane & 3;
+            int pa[4], pb[4];              // offsets in shared memory
+            bool have[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int q = 4 * e + q4, at = (q < full ? q : q - full) * ld + par;
+                have[e] = q < 2 * full;
+                pa[e] = have[e] ? (q < full ? lay.u() : lay.w()) + at : 0;
+                pb[e] = have[e] ? (q < full ? lay.w() : lay.u()) + at : 0;
+            }
+            for (int m0 = mw; m0 < cnt; m0 += 8 * kTriWarps) {
+                const int lb = rank + CL * min(m0 + kTriWarps * g, cnt - 1);
+                double bf[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) bf[e] = have[e] ? -sm[pb[e] + lb] : 0.0;
+                const int mc0 = m0 + 2 * kTriWarps * q4, mc1 = mc0 + kTriWarps;
+                double* c0 = t.A + (size_t)(rank + CL * min(mc0, cnt - 1)) * n;
+                double* c1 = t.A + (size_t)(rank + CL * min(mc1, cnt - 1)) * n;
+                double s0 = 0.0, s1 = 0.0;
+                auto fetch = [&](int R, double (&x)[8][2]) {
+                    if (R + 64 <= n) {
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            x[u][0] = c0[R + g + 8 * u];
+                            x[u][1] = c1[R + g + 8 * u];
+                        }
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            x[u][0] = c0[min(R + g + 8 * u, n - 1)];
+                            x[u][1] = c1[min(R + g + 8 * u, n - 1)];
+                        }
+                    }
+                };
+                auto apply_at = [&](int R, double (&x)[8][2]) {
+                    const int last = n - 1;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (4 * e < 2 * full) {
+#pragma unroll
+                            for (int u = 0; u < 8; ++u)
+                                nrg::cta_dmma(x[u][0], x[u][1], sm[pa[e] + min(R + g + 8 * u, last)], bf[e]);
+                        }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const int i = R + g + 8 * u;
+                        if (i < n) {
+                            if (mc0 < cnt) c0[i] = x[u][0];
+                            if (mc1 < cnt) c1[i] = x[u][1];
+                            const double xv = fin ? 0.0 : xs[i];
+                            s0 = fma(x[u][0], xv, s0);
+                            s1 = fma(x[u][1], xv, s1);
+                        }
+                    }
+                    if (R == r0 && g == 0 && !fin) {   // row k + 1
+                        if (mc0 < cnt) rowv[mc0] = x[0][0];
+                        if (mc1 < cnt) rowv[mc1] = x[0][1];
+                    }
+                };
+                double x[8][2], y[8][2];
+                fetch(r0, x);
+                for (int R = r0; R < n; R += 128) {
+                    if (R + 64 < n) fetch(R + 64, y);
+                    apply_at(R, x);
+                    if (R + 128 < n) fetch(R + 128, x);
+                    if (R + 64 < n) apply_at(R + 64, y);
+                }
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    s0 += __shfl_xor_sync(kAll, s0, o);
+                    s1 += __shfl_xor_sync(kAll, s1, o);
+                }
+                if (g == 0 && !fin) {
+                    if (mc0 < cnt) part[mc0] = s0;
+                    if (mc1 < cnt) part[mc1] = s1;
+                }
+            }
+        } else {
+            // three columns at a time in parts of 256 rows, 16-byte loads of row pairs, the next
+            // part's loads in flight.  Pairs beyond the end repeat the last whole one against a
+            // zero; the last row is taken by itself when it has no partner.
+            const int rs = (k + 1) - ((k + 1 + par) & 1);
+            const int pend = rs + 2 * ((n - rs) / 2);                  // end of the whole pairs
+            for (int m0 = mw; m0 < cnt; m0 += 3 * kTriWarps) {
+                const double* col[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    col[c] = t.A + (size_t)(rank + CL * min(m0 + kTriWarps * c, cnt - 1)) * n + 2 * lane;
+                auto fetch = [&](int R, double2 (&x)[3][4]) {
+                    if (R + 256 <= pend) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) x[c][u] = *reinterpret_cast<const double2*>(col[c] + R + 64 * u);
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int i = min(R + 64 * u, pend - 2 - 2 * lane);
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) x[c][u] = *reinterpret_cast<const double2*>(col[c] + i);
+                        }
+                    }
+                };
+                double sum[4] = {0.0, 0.0, 0.0, 0.0};
+                auto use = [&](int R, const double2 (&x)[3][4]) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int i = R + 64 * u + 2 * lane;
+                        double2 xv = make_double2(0.0, 0.0);
+                        if (i < pend) xv = *reinterpret_cast<const double2*>(xs + i);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) sum[c] = fma(x[c][u].y, xv.y, fma(x[c][u].x, xv.x, sum[c]));
+                    }
+                };
+                double2 x[3][4], y[3][4];
+                fetch(rs, x);
+                if (lane == 0) {               // row k + 1 of these columns
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                        if (m0 + kTriWarps * c < cnt) rowv[m0 + kTriWarps * c] = rs == k + 1 ? x[c][0].x : x[c][0].y;
+                    if (pend < n)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) sum[c] = col[c][n - 1] * xs[n - 1];
+                }
+                for (int R = rs; R < pend; R += 512) {
+                    if (R + 256 < pend) fetch(R + 256, y);
+                    use(R, x);
+                    if (R + 512 < pend) fetch(R + 512, x);
+                    if (R + 256 < pend) use(R + 256, y);
+                }
+                const double tot = sum4(sum, lane);
+                const int mc = m0 + kTriWarps * ((lane >> 3) & 3);
+                if ((lane & 7) == 0 && (lane >> 3) < 3 && mc < cnt) part[mc] = tot;
+            }
+        }
+        if (!fin) {
+            // the warp's part of u.y
+            __syncwarp();
+            double yv = 0.0;
+            for (int m = mw + kTriWarps * lane; m < cnt; m += 32 * kTriWarps) yv = fma(part[m], xs[rank + CL * m], yv);
+            yv = bfly(yv);
+            if (lane == 0) pw[warp] = yv;
+            // the kept updates' products with the new column: every block takes a run of rows
+            if (warp < next) {
+                const double *uq = U + warp * ld + par, *wq = W + warp * ld + par;
+                double d1 = 0.0, d2 = 0.0;
+                const int run = (n - k - 2 + CL - 1) / CL, end = min(n, k + 2 + (rank + 1) * run);
+                for (int i = k + 2 + rank * run + lane; i < end; i += 32) {
+                    const double x = xs[i];
+                    d1 = fma(wq[i], x, d1);
+                    d2 = fma(uq[i], x, d2);
+                }
+                d1 = bfly(d1);
+                d2 = bfly(d2);
+                if (lane == 0) tsum[8 * warp] = d1, tsum[8 * warp + 1] = d2;
+            }
+        }
+        if (fin) break;
+        step_sync();
+        const double un = sc[kScale];
+        if (un != 1.0) {
+            // the rare normalised reflector: what was formed with the column takes the factor
+            for (int i = k + 2 + tid; i < n; i += kTriRows) U[nw + i] *= un;
+            for (int m = tid; m < cnt; m += kTriRows) part[m] *= un;
+            if (tid < kTriWarps) pw[tid] *= un * un;
+            if (tid < 2 * next) tsum[8 * (tid >> 1) + (tid & 1)] *= un;
+            step_sync();
+        }
+        // ---- 3. sums, row k + 1 and the parts of the dot products to every block ----
+        const unsigned bar = bar0 + 8 * (b ^ 1);
+        // a warp sends 32 columns to one block at a time
+        const int mB = first_own(k + 1);
+        const int parts = (cnt - mB + 31) / 32;
+        for (int e = warp; e < CL * parts; e += kTriWarps) {
+            const int r = e % CL, m = mB + 32 * (e / CL) + lane;
+            if (m >= cnt) continue;
+            send16(map_rank(buf0 + 16 * ((b ^ 1) * lay.nr + rank * lay.cols + m), to0 + r), part[m], rowv[m],
+                   map_rank(bar, to0 + r));
+        }
+        // after the updates went in, the new column is the first one kept
+        if (apply)
+            for (int i = k + 2 + tid; i < n; i += kTriRows) U[par + i] = U[nw + i];
+        np = next;
+    }
+}
+
+template <int CL>
+__global__ void __launch_bounds__(kTriThreads, 1) k_tri_stream(const StreamTask* __restrict__ tasks, int* status) {
+    extern __shared__ __align__(16) double tri_sm[];
+    const StreamTask t = tasks[blockIdx.x];
+    const int tid = threadIdx.x, warp = tid >> 5;
+    double* sm = tri_sm;
+    {
+        const StreamLayout lay(t.n, CL, t.keep);
+        for (int i = tid; i < lay.doubles(CL); i += kTriThreads) sm[i] = 0.0;
+        __syncthreads();
+        // step 0 reads y = 0 and column 0
+        for (int i = tid; i < t.n; i += kTriThreads) sm[lay.buf() + 2 * ((i % CL) * lay.cols + i / CL) + 1] = t.A[i];
+        if (tid == 0) {
+            const unsigned bar = smem_addr(sm + lay.bar(CL));
+            bar_init(bar);
+            bar_init(bar + 8);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+    }
+    __syncthreads();
+    // no block stores a reflector before every block has read column 0
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    unsigned cta;
+    asm("mov.u32 %0, %cluster_ctarank;" : "=r"(cta));
+    const unsigned to0 = cta - (unsigned)t.rank;
+    if (warp < kTriWarps) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMatrixRegs));
+        stream_steps<CL>(t, sm, to0, status);
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kNormRegs));
+        if (warp == kTriWarps) stream_norm_steps<CL>(t, sm, to0);
+    }
+    // no block leaves while another may still write its shared memory
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // the sectors of order <= 128, one block each: D, E and tau go where k_syev reads them
 __global__ void __launch_bounds__(kTriThreads, 1) k_tri_small(const SyevSector* __restrict__ secs, double* eigbuf,
                                                              double* wsd, int* status) {
@@ -558,6 +1035,7 @@ __global__ void __launch_bounds__(kTriThreads, 1) k_tri_small(const SyevSector* 
     else tri_run<Plan0, false>(t, tri_sm, 0, status);
 }
 
+constexpr long long kSmemMax = 232448;   // 227 KB, the most one block may use
 constexpr int kPlans = 6, kPlanCL[kPlans] = {1, 2, 4, 8, 8, 16};
 constexpr int kPlanMax[kPlans] = {Plan0::kMax, Plan1::kMax, Plan2::kMax, Plan3::kMax, Plan4::kMax, Plan5::kMax};
 constexpr size_t kPlanBytes[kPlans] = {Plan0::kBytes, Plan1::kBytes, Plan2::kBytes, Plan3::kBytes, Plan4::kBytes,
@@ -582,6 +1060,7 @@ int launch_clusters(nrg_context* ctx, const TriTask* d_tasks, int blocks, size_t
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
     cluster_config<MAXCL>(&cfg, at, blocks, smem, ctx->stream);
+    if (MAXCL > 8) NRG_CUDA_TRY(cudaFuncSetAttribute(k_tri_res<MAXCL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     NRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tri_res<MAXCL>, d_tasks, d_status));
     ctx->launches++;
     return NRG_OK;
@@ -611,6 +1090,50 @@ int tri_resident_max() {
         known[dev].store(m);
     }
     return m;
+}
+
+bool tri_wide_clusters() { return tri_resident_max() == kPlanMax[kPlans - 1]; }
+
+int tri_stream_max() {
+    static const int m = [] {
+        int n = 2;
+        while (8LL * StreamLayout(n + 1, 16, 1).doubles(16) <= kSmemMax) ++n;
+        return n;
+    }();
+    return m;
+}
+
+int tri_stream(nrg_context* ctx, const std::vector<TriItem>& items, int CL, DevBuf& buf) {
+    if (items.empty()) return NRG_OK;
+    std::vector<StreamTask> tasks;
+    size_t smem = 0;
+    for (const TriItem& it : items) {
+        int keep = kStreamSlots;
+        while (keep > 1 && 8LL * StreamLayout(it.n, CL, keep).doubles(CL) > kSmemMax) --keep;
+        smem = std::max(smem, sizeof(double) * (size_t)StreamLayout(it.n, CL, keep).doubles(CL));
+        for (int r = 0; r < CL; ++r) tasks.push_back(StreamTask{it.A, it.D, it.E, it.TAU, it.n, it.stop, r, keep});
+    }
+    if (smem > (size_t)kSmemMax) {
+        nrg_set_error_message("order %d exceeds the streamed tridiagonalisation", items[0].n);
+        return NRG_ERR_TOO_LARGE;
+    }
+    NRG_TRY(buf.ensure(sizeof(StreamTask) * tasks.size()));
+    NRG_TRY(h2d_async(ctx, buf.p, tasks.data(), sizeof(StreamTask) * tasks.size()));
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    const int blocks = (int)tasks.size();
+    if (CL == 16) {
+        NRG_TRY(raise_smem_limit((const void*)k_tri_stream<16>, smem));
+        NRG_CUDA_TRY(cudaFuncSetAttribute(k_tri_stream<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cluster_config<16>(&cfg, at, blocks, smem, ctx->stream);
+        NRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tri_stream<16>, (const StreamTask*)buf.as<StreamTask>(), ctx->d_status.as<int>()));
+    } else {
+        NRG_TRY(raise_smem_limit((const void*)k_tri_stream<8>, smem));
+        cluster_config<8>(&cfg, at, blocks, smem, ctx->stream);
+        NRG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tri_stream<8>, (const StreamTask*)buf.as<StreamTask>(), ctx->d_status.as<int>()));
+    }
+    ctx->launches++;
+    return NRG_OK;
 }
 
 int tri_resident(nrg_context* ctx, const std::vector<TriItem>& items, DevBuf& buf) {

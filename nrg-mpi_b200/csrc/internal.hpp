@@ -112,7 +112,7 @@ struct Sectors {
 // the context
 // ------------------------------------------------------------------------------------
 struct Scratch {
-    DevBuf b[48];
+    DevBuf b[50];
 };
 
 }  // namespace nrg
@@ -279,16 +279,21 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& secs, double* d_
                cudaEvent_t evals_ready = nullptr);
 constexpr int kLargeSector = 128;
 
-// tridiagonalisation with the matrix resident on chip (eig_tri.cu): D, E, tau and the
-// reflectors (below the subdiagonal of A) of every item, on ctx->stream; orders 2 ..
-// tri_resident_max()
+// tridiagonalisation (eig_tri.cu) on ctx->stream: D, E, tau and the reflectors (below the
+// subdiagonal of A) of every item.  tri_resident: the matrix on chip, orders 2 ..
+// tri_resident_max().  tri_stream: the first `stop` columns of a larger one (up to
+// tri_stream_max(), lda = n) by clusters of CL = 8 or 16 blocks; the trailing block is left
+// updated for tri_resident.
 struct TriItem {
     double* A;             // full symmetric storage, leading dimension lda
     double *D, *E, *TAU;
-    int n, lda;
+    int n, lda, stop;
 };
 int tri_resident_max();
+bool tri_wide_clusters();   // clusters of 16 blocks can be placed
 int tri_resident(nrg_context* ctx, const std::vector<TriItem>& items, DevBuf& tasks);
+int tri_stream_max();
+int tri_stream(nrg_context* ctx, const std::vector<TriItem>& items, int CL, DevBuf& tasks);
 
 // ---- kernels (kernels.cu) ------------------------------------------------------------
 int run_assemble(nrg_context* ctx, int iteration, const Sectors& S, const SyevSector* d_secs,

@@ -1,7 +1,7 @@
-"""The on-chip tridiagonalisation at the edges of its plans (orders 64, 128, 160, 256, 320,
-384, 512 and one beyond each, the smallest orders, and orders whose first columns go
-through the panel kernel), through the entries that use it: nrg_diagonalization on a
-synthetic iteration and nrg_block_eigh_noalloc.
+"""The tridiagonalisation at the edges of its plans (on chip: orders 64, 128, 160, 256, 320,
+384, 512 and one beyond each, the smallest orders; streamed: one column, fewer and more
+columns than updates are kept back, and orders that keep fewer back), through the entries
+that use it: nrg_diagonalization on a synthetic iteration and nrg_block_eigh_noalloc.
 
 Tolerances: a backward stable solver's residual and loss of orthogonality are a small
 multiple of n eps (times the norm of H for the residual); 20 n eps is allowed, for the
@@ -55,7 +55,7 @@ def test_block(n, kind):
     check(H, E.cpu().numpy(), V.cpu().numpy().T)
 
 
-@pytest.mark.parametrize("n", [129, 159, 160, 161, 255, 256, 257, 319, 320, 321, 383, 384, 385, 511, 512, 513, 545, 640])
+@pytest.mark.parametrize("n", [129, 159, 160, 161, 255, 256, 257, 319, 320, 321, 383, 384, 385, 511, 512, 513, 545, 640, 1500, 2100])
 def test_sector(n, ctx_factory):
     """One iteration whose old states are a sector of n // 2 and one of n - n // 2 states that
     f-dagger-up connects: the new sectors have orders n, n // 2 and n - n // 2."""
