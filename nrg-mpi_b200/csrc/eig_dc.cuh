@@ -147,9 +147,13 @@ __device__ __forceinline__ int last_below(const unsigned (&w)[4], int i) {   // 
     return -1;
 }
 
-// Root j of 1 + rho sum_i zz_i^2 / (dd_i - lambda) as in secular_root (eig_common.cuh), with
-// the evaluation at the middle of the interval used for the choice of the origin and for
-// the first step.
+// Root j of 1 + rho sum_i zz_i^2 / (dd_i - lambda) = 0 (rho > 0, dd ascending, zz != 0),
+// returned as lambda = dd[org] + tau with org the pole nearer to the root, so that every
+// difference dd_i - lambda = (dd_i - dd[org]) - tau keeps full relative accuracy.
+// Iteration: the two-pole rational model of the secular function (the poles bounding the
+// root carry the near terms, Bunch-Nielsen-Sorensen), solved as a quadratic, kept inside a
+// bisection bracket; at most 100 steps.  The evaluation at the middle of the interval
+// serves the choice of the origin and the first step.
 template <class G>
 __device__ void leaf_root(const G& g, int first, int K, const double* dd, const double* zz, double rho, int j, int* org,
                           double* tau, int* status) {

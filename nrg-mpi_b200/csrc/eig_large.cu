@@ -33,7 +33,8 @@ constexpr int CB = 32;        // columns per block in the symmetric matrix-vecto
 
 struct LSec {
     long long a_off, e_off, w_off, i_off;
-    int n, pad;
+    int n;
+    int z_sel;   // where the divide and conquer leaves the eigenvectors: 0 Z, 2 Qt (in n x n)
 };
 
 // workspace per sector: Z, U, Qt (n x n each), the panel V | W (n x 2 NB), y, the D&C
@@ -45,7 +46,7 @@ long long lws_doubles(long long n) {
 long long lws_ints(long long n) { return 12 * n + 64; }
 
 struct LView {
-    double *A, *Z, *U, *Qt, *VW, *y, *vec, *D, *E, *TAU, *R;
+    double *A, *Z, *U, *Qt, *ZV, *VW, *y, *vec, *D, *E, *TAU, *R;   // ZV: the eigenvectors of T
     int* I;
     Scratch S;
     int n;
@@ -60,6 +61,7 @@ __device__ LView lview(const LSec& s, double* eigbuf, double* wsd, int* wsi) {
     v.Z = W;
     v.U = W + sq;
     v.Qt = W + 2 * sq;
+    v.ZV = W + s.z_sel * sq;
     v.VW = W + 3 * sq;
     v.y = v.VW + 2LL * NB * n;
     v.vec = v.y + n;
@@ -231,76 +233,303 @@ __global__ void __launch_bounds__(kLeafThreads) k_dc_low(const LSec* __restrict_
     dc_leaf(c0, min(DC_LOW, L.n - c0), L.n, L.D, L.E, L.Z, sm, status);
 }
 
+// Merges beyond DC_LOW rows, all merges of one level at once, in five launches: poles and
+// deflation (a block per merge), secular roots, Gu-Eisenstat z with the order of the results,
+// rank-one eigenvectors with the deflated columns (a warp per item), and the eigenvector
+// update as one grouped GEMM.  The children's blocks are read from one of two buffers and
+// the merged block is written to the other, so nothing is copied back; the rows of the
+// rank-one eigenvectors are the children's columns, so that the update is two products of
+// half the inner length per merge and no operand is gathered.  Before: ten launches per
+// level, the deflation scan on one thread (230..315 us at 1225 rows) and the update over
+// the children's zero blocks.
 struct Merge {
-    int sec, a, mid, b;
-    // block ranges of the parallel phases for the three thread mappings: one thread per
-    // item (kMapItem), one warp per item (kMapWarp), one thread per few matrix entries
-    // of the nn x nn merged block (kMapWide)
-    int blk0[3], nblk[3];
+    int sec, a, mid, b;   // mid == b: a block without a partner at this level
+    int blk0, nblk;       // blocks of the warp-per-item launches
 };
-constexpr int kMapItem = 0, kMapWarp = 1, kMapWide = 2;
-constexpr int kWideItems = 8;   // matrix entries per thread in kMapWide
 
-__device__ int find_merge(const Merge* ms, int nm, int map) {
+__device__ int find_merge(const Merge* ms, int nm) {
     int lo = 0, hi = nm - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (ms[mid].blk0[map] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+        if (ms[mid].blk0 <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
 
-__global__ void __launch_bounds__(512) k_dc_prep(const LSec* __restrict__ secs, const Merge* __restrict__ ms,
-                                                 double* eigbuf, double* wsd, int* wsi) {
-    __shared__ double red[32];
-    const Merge m = ms[blockIdx.x];
-    LView L = lview(secs[m.sec], eigbuf, wsd, wsi);
-    merge_prep(BlockG{}, m.a, m.mid, m.b, L.n, L.Z, L.D, L.E, L.S, red);
+constexpr int kPrepThreads = 512;
+constexpr size_t kPrepSmem = 200 * 1024;   // four doubles per row in shared memory up to 6,400 rows
+
+// exclusive scans over the block of an int per thread: the sum, or the maximum with -1 first
+__device__ int block_scan(int v, bool maximum, int* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x = maximum ? max(x, y) : x + y;
+    }
+    __syncthreads();
+    if (lane == 31) red[warp] = x;
+    __syncthreads();
+    int base = maximum ? -1 : 0;
+    for (int w = 0; w < warp; ++w) base = maximum ? max(base, red[w]) : base + red[w];
+    const int y = __shfl_up_sync(0xffffffffu, x, 1);
+    const int before = lane == 0 ? (maximum ? -1 : 0) : y;
+    return maximum ? max(base, before) : base + before;
 }
 
-// phase 1 roots, 2 zhat, 3 rank-one vectors + values (one warp per root / entry / column),
-// 4 final order + GEMM index lists (one thread per item), 5 deflated copies, 6 copy back
-// (one thread per few entries)
-__global__ void __launch_bounds__(TPB) k_dc_phase(const LSec* __restrict__ secs, const Merge* __restrict__ ms,
-                                                  int nm, int phase, double* eigbuf, double* wsd, int* wsi,
-                                                  int* status) {
-    const int map = phase <= 3 ? kMapWarp : (phase == 4 ? kMapItem : kMapWide);
-    const int mi = find_merge(ms, nm, map);
-    const Merge m = ms[mi];
+// z, merge order, poles and deflation of one merge.  Deflated entries: negligible z, found in
+// parallel, and the first of a pair of close poles, rotated into the second.  Whether a pair
+// is close depends on its predecessor only through a rotation, so one thread visits just
+// the entries that are close to the unrotated one before them, and what follows each as
+// long as rotations go on.  df: the rotated entries in the order of the rotations, then the
+// negligible ones; chain starts in `nd`'s tail are not needed: rotation r continues the
+// one before when it shares its entry.
+__global__ void __launch_bounds__(kPrepThreads) k_dc_prep(const LSec* __restrict__ secs, const Merge* __restrict__ ms,
+                                                          long long z_off, double* eigbuf, double* wsd, int* wsi) {
+    extern __shared__ __align__(16) double psm[];
+    __shared__ double red[32];
+    __shared__ int ired[32];
+    __shared__ int nflag, nrots;
+    const Merge m = ms[blockIdx.x];
+    if (m.mid == m.b) return;
     LView L = lview(secs[m.sec], eigbuf, wsd, wsi);
-    const int t = ((int)blockIdx.x - m.blk0[map]) * blockDim.x + threadIdx.x;
-    const int T = m.nblk[map] * blockDim.x;
-    const WarpLanes wl{(int)(threadIdx.x & 31)};
-    switch (phase) {
-        case 1: merge_roots(t >> 5, T >> 5, m.a, m.mid, L.E, L.S, status, wl); break;
-        case 2: merge_zhat(t >> 5, T >> 5, m.a, m.mid, L.E, L.S, wl); break;
-        case 3:
-            merge_ucols(t >> 5, T >> 5, m.a, L.n, L.S, L.U, wl);
-            merge_vals(t, T, m.a, m.b, L.S);
-            break;
-        case 4: {
-            merge_rank(t, T, m.a, m.b, L.S);
-            const int K = L.S.mk[m.a];
-            // gathered columns of Z for the GEMM: a + perm[nd[q]] (ra reused after prep)
-            for (int q = t; q < K; q += T) L.S.ra[m.a + q] = m.a + L.S.perm[m.a + L.S.nd[m.a + q]];
-            break;
+    const int n = L.n, a = m.a, nn = m.b - m.a, n1 = m.mid - m.a, t = threadIdx.x;
+    const double* Z = L.Z + z_off * n * n;
+    const bool in_smem = 4 * sizeof(double) * (size_t)nn <= kPrepSmem;
+    double* Dm = in_smem ? psm : L.D + a;
+    double* z = in_smem ? psm + nn : L.S.z + a;
+    double* ds = in_smem ? psm + 2 * nn : L.S.ds + a;
+    double* zs = in_smem ? psm + 3 * nn : L.S.zs + a;
+    int *perm = L.S.perm + a, *nd = L.S.nd + a, *df = L.S.df + a, *flag = L.S.org + a, *kind = L.S.pos + a;
+    const double beta = L.E[m.mid - 1], rho = 2.0 * fabs(beta), sg = beta >= 0.0 ? 1.0 : -1.0;
+    for (int i = t; i < nn; i += kPrepThreads) {
+        if (in_smem) Dm[i] = L.D[a + i];
+        z[i] = (i < n1 ? Z[(size_t)(m.mid - 1) + (size_t)(a + i) * n] : sg * Z[(size_t)m.mid + (size_t)(a + i) * n]) *
+               0.70710678118654752440;
+    }
+    if (t == 0) nflag = nrots = 0;
+    __syncthreads();
+    // stable merge order of the two ascending halves (first half wins ties)
+    double dm = 0.0, zm = 0.0;
+    for (int i = t; i < nn; i += kPrepThreads) {
+        const bool one = i < n1;
+        const double v = Dm[i];
+        int lo = 0, hi = one ? nn - n1 : n1;
+        const double* o = one ? Dm + n1 : Dm;
+        while (lo < hi) {
+            const int x = (lo + hi) >> 1;
+            if (one ? o[x] < v : o[x] <= v) lo = x + 1; else hi = x;
         }
-        case 5: merge_deflated(t, T, m.a, m.b, L.n, L.Z, L.Qt, L.S); break;
-        case 6: merge_copyback(t, T, m.a, m.b, L.n, L.Z, L.D, L.Qt, L.S); break;
-        default: break;
+        const int r = (one ? i : i - n1) + lo;
+        perm[r] = i;
+        ds[r] = v;
+        zs[r] = z[i];
+        dm = fmax(dm, fabs(v));
+        zm = fmax(zm, fabs(z[i]));
+    }
+    const double tol = 8.0 * kEps * block_max(fmax(dm, rho * zm), red);
+    __syncthreads();
+    // a run of entries per thread: kind 0 kept, 1 negligible, 2 rotated out
+    const int run = (nn + kPrepThreads - 1) / kPrepThreads, r0 = min(t * run, nn), r1 = min(r0 + run, nn);
+    int last = -1;
+    for (int r = r0; r < r1; ++r) {
+        const bool live = rho * fabs(zs[r]) > tol;
+        kind[r] = live ? 0 : 1;
+        if (live) last = r;
+    }
+    int prev = block_scan(last, true, ired);
+    auto close_to = [&](double zj, double dj, double zl, double dl) {
+        // |(d_j - d_l) c s| <= tol with c = z_j / r, s = -z_l / r, r^2 = z_j^2 + z_l^2
+        return fabs(dj - dl) * fabs(zj * zl) <= tol * fma(zj, zj, zl * zl);
+    };
+    int mine = 0;
+    {
+        int l = prev;
+        for (int r = r0; r < r1; ++r)
+            if (kind[r] == 0) {
+                if (l >= 0 && close_to(zs[r], ds[r], zs[l], ds[l])) ++mine;
+                l = r;
+            }
+    }
+    int at = block_scan(mine, false, ired);
+    {
+        int l = prev;
+        for (int r = r0; r < r1; ++r)
+            if (kind[r] == 0) {
+                if (l >= 0 && close_to(zs[r], ds[r], zs[l], ds[l])) flag[at++] = r;
+                l = r;
+            }
+    }
+    if (t == kPrepThreads - 1) nflag = at;
+    __syncthreads();
+    if (t == 0 && nflag > 0) {
+        int nrot = 0, done = -1;
+        for (int f = 0; f < nflag; ++f) {
+            int j = flag[f];
+            if (j <= done) continue;
+            int l = j - 1;
+            while (kind[l] != 0) --l;           // the entry it is close to is still there: it was not visited
+            double zl = zs[l], dl = ds[l];
+            for (;;) {
+                const double zj = zs[j], dj = ds[j];
+                done = j;
+                if (!close_to(zj, dj, zl, dl)) break;
+                const double r = hypot(zj, zl), c_ = zj / r, s_ = -zl / r;
+                L.S.ra[a + nrot] = perm[l];
+                L.S.rb[a + nrot] = perm[j];
+                L.S.rc[a + nrot] = c_;
+                L.S.rs[a + nrot] = s_;
+                df[nrot++] = l;
+                const double tn = dl * c_ * c_ + dj * s_ * s_, dn = dl * s_ * s_ + dj * c_ * c_;
+                zs[j] = zl = r;
+                zs[l] = 0.0;
+                ds[j] = dl = dn;
+                ds[l] = tn;
+                kind[l] = 2;
+                l = j;
+                do ++j; while (j < nn && kind[j] != 0);
+                if (j >= nn) break;
+            }
+        }
+        nrots = nrot;
+    }
+    __syncthreads();
+    int nk = 0, nz = 0;
+    for (int r = r0; r < r1; ++r) {
+        nk += kind[r] == 0;
+        nz += kind[r] == 1;
+    }
+    int qk = block_scan(nk, false, ired), qz = block_scan(nz, false, ired) + nrots;
+    for (int r = r0; r < r1; ++r) {
+        if (kind[r] == 0) {
+            nd[qk] = perm[r];
+            L.S.dd[a + qk] = ds[r];
+            L.S.zz[a + qk] = zs[r];
+            ++qk;
+        } else if (kind[r] == 1) {
+            df[qz++] = r;
+        }
+    }
+    if (t == kPrepThreads - 1) {
+        L.S.mk[a] = qk;             // roots
+        L.S.mr[a] = nrots;
+        L.S.mf[a] = qk + nrots;     // columns of the eigenvector update
+    }
+    __syncthreads();
+    // deflated values follow the roots; df becomes the child column of the entry
+    const int K = L.S.mk[a];
+    for (int q = t; q < nn - K; q += kPrepThreads) {
+        const int r = df[q];
+        L.S.vals[a + K + q] = ds[r];
+        df[q] = perm[r];
     }
 }
 
-// scatter columns a + pos[j] of the nondeflated eigenvectors (rb reused)
-__global__ void k_dc_poscols(const LSec* __restrict__ secs, const Merge* __restrict__ ms, int nm,
-                             double* eigbuf, double* wsd, int* wsi) {
-    const int mi = find_merge(ms, nm, kMapItem);
-    const Merge m = ms[mi];
+// the 32 lanes of a warp on one item
+struct WarpItem {
+    static constexpr int kPer = 32;
+    __device__ double sum(double v) const {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    }
+    __device__ double prod(double v) const {
+        for (int o = 16; o > 0; o >>= 1) v *= __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    }
+};
+
+// phase 1 secular roots, 2 z and places of the results, 3 rank-one eigenvectors and deflated
+// columns: one warp per item
+template <int PHASE>
+__global__ void __launch_bounds__(TPB) k_dc_items(const LSec* __restrict__ secs, const Merge* __restrict__ ms, int nm,
+                                                  long long z_in, long long z_out, double* eigbuf, double* wsd, int* wsi,
+                                                  int* status) {
+    const Merge m = ms[find_merge(ms, nm)];
     LView L = lview(secs[m.sec], eigbuf, wsd, wsi);
-    const int t = ((int)blockIdx.x - m.blk0[kMapItem]) * blockDim.x + threadIdx.x;
-    const int T = m.nblk[kMapItem] * blockDim.x;
-    const int K = L.S.mk[m.a];
-    for (int j = t; j < K; j += T) L.S.rb[m.a + j] = m.a + L.S.pos[m.a + j];
+    const int n = L.n, a = m.a, nn = m.b - m.a, lane = threadIdx.x & 31;
+    const int e = ((int)blockIdx.x - m.blk0) * (TPB / 32) + (threadIdx.x >> 5);
+    if (e >= nn) return;
+    const WarpItem g;
+    const bool alone = m.mid == m.b;
+    const int K = alone ? 0 : L.S.mk[a];
+    const double rho = 2.0 * fabs(L.E[m.mid - 1]);
+    const double *dd = L.S.dd + a, *zz = L.S.zz + a, *tau = L.S.tau + a;
+    const int* org = L.S.org + a;
+    if constexpr (PHASE == 1) {
+        if (e < K) {
+            leaf_root(g, lane, K, dd, zz, rho, e, L.S.org + a + e, L.S.tau + a + e, status);
+            __syncwarp();
+            if (lane == 0) L.S.vals[a + e] = dd[org[e]] + tau[e];
+        }
+    } else if constexpr (PHASE == 2) {
+        if (alone) return;
+        if (e < K) {
+            const double di = dd[e];
+            double p = 1.0;
+            for (int j = lane; j < K - 1; j += 32) p *= quotient((di - dd[org[j]]) - tau[j], di - dd[j < e ? j : j + 1]);
+            p = g.prod(p) * quotient(-((di - dd[org[K - 1]]) - tau[K - 1]), rho);
+            if (lane == 0) L.S.zh[a + e] = copysign(root_of(fmax(p, 0.0)), zz[e]);
+        }
+        // place in ascending order, ties in list order (roots, then deflated values)
+        const double* vals = L.S.vals + a;
+        const double v = vals[e];
+        int r = 0;
+        for (int f = lane; f < nn; f += 32) {
+            const double w = vals[f];
+            r += (w < v) || (w == v && f < e);
+        }
+        r = __reduce_add_sync(0xffffffffu, r);
+        if (lane == 0) {
+            L.S.pos[a + e] = r;
+            L.D[a + r] = v;
+        }
+    } else {
+        const double* Z = L.Z + z_in * n * n;
+        double* Q = L.Z + z_out * n * n;
+        const int N = alone ? 0 : L.S.mf[a];
+        const int *nd = L.S.nd + a, *df = L.S.df + a;
+        if (e >= N) {
+            // a column that only moves: a deflated one, or any of a block without a partner
+            const int src = alone ? e : df[e - K], dst = alone ? e : L.S.pos[a + e];
+            const bool one = a + src < m.mid;
+            for (int i = a + lane; i < m.b; i += 32)
+                Q[(size_t)i + (size_t)(a + dst) * n] = (i < m.mid) == one ? Z[(size_t)i + (size_t)(a + src) * n] : 0.0;
+            return;
+        }
+        double* uc = L.U + (size_t)a + (size_t)(a + e) * n;
+        for (int q = lane; q < nn - K; q += 32) uc[df[q]] = 0.0;
+        if (e < K) {
+            double q = 0.0;
+            const double dj = dd[org[e]], tj = tau[e];
+            for (int i = lane; i < K; i += 32) {
+                const double u = quotient(L.S.zh[a + i], (dd[i] - dj) - tj);
+                uc[nd[i]] = u;
+                q = fma(u, u, q);
+            }
+            q = rsqrt(g.sum(q));
+            for (int i = lane; i < K; i += 32) uc[nd[i]] *= q;
+        } else {
+            for (int i = lane; i < K; i += 32) uc[nd[i]] = 0.0;
+            __syncwarp();
+            if (lane == 0) uc[df[e - K]] = 1.0;
+        }
+        const int nrot = L.S.mr[a];
+        if (nrot == 0) return;
+        __syncwarp();
+        // rotated columns: the rows take the rotations, last one first; rotations that share
+        // no entry run side by side (a chain shares each entry with the next rotation)
+        const int *ra = L.S.ra + a, *rb = L.S.rb + a;
+        for (int r0 = lane; r0 < nrot; r0 += 32) {
+            if (r0 + 1 < nrot && ra[r0 + 1] == rb[r0]) continue;   // not the last of its chain
+            for (int r = r0; r >= 0; --r) {
+                const double c_ = L.S.rc[a + r], s_ = L.S.rs[a + r], x = uc[ra[r]], y = uc[rb[r]];
+                uc[ra[r]] = fma(c_, x, -s_ * y);
+                uc[rb[r]] = fma(s_, x, c_ * y);
+                if (r == 0 || ra[r] != rb[r - 1]) break;
+            }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------
@@ -476,7 +705,7 @@ __global__ void __launch_bounds__(256, 1) k_bt_apply(const LSec* __restrict__ se
     const int wr = 8 * warp;                // this warp's slice of reflectors / rows
     for (int j = 0; j < CBK; ++j)
         for (int row = tid; row < n; row += 256)
-            Zs[(size_t)j * ldz + row] = j < nc ? L.Z[(size_t)row + (size_t)(c0 + j) * n] : 0.0;
+            Zs[(size_t)j * ldz + row] = j < nc ? L.ZV[(size_t)row + (size_t)(c0 + j) * n] : 0.0;
     const int qmax = (n - 2) / NBB;
     // the load sequence: step t of panel q is a V chunk (t < C: for W; t > C: for the
     // update, chunk t - C - 1) or T (t == C), with C = ceil(mr / 64) chunks per pass
@@ -624,7 +853,9 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         secs[s].a_off = in[s].a_off;
         secs[s].e_off = in[s].e_off;
         secs[s].n = in[s].n;
-        secs[s].pad = 0;
+        int levels = 0;
+        for (int w = DC_LOW; w < in[s].n; w *= 2) ++levels;
+        secs[s].z_sel = levels % 2 ? 2 : 0;
         secs[s].w_off = wd;
         secs[s].i_off = wi;
         wd += lws_doubles(in[s].n);
@@ -748,60 +979,57 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         ctx->launches++;
         NRG_CUDA_TRY(cudaGetLastError());
     }
+    // the eigenvectors alternate between Z and Qt from level to level (in units of n x n)
+    long long z_in = 0, z_out = 2;
+    NRG_TRY(raise_smem_limit((const void*)k_dc_prep, kPrepSmem));
     for (int s = DC_LOW; s < maxn; s *= 2) {
         std::vector<Merge> ms;
-        int blk[3] = {0, 0, 0};
+        std::vector<GemmProblem> probs;
+        int blk = 0, widest = 0;
         for (int x = 0; x < ns; ++x) {
             const int n = secs[x].n;
-            for (int a = 0; a + s < n; a += 2 * s) {
+            for (int a = 0; a < n && s < n; a += 2 * s) {
                 Merge m;
-                m.sec = x; m.a = a; m.mid = a + s; m.b = std::min(a + 2 * s, n);
-                const long long nn = m.b - m.a;
-                m.nblk[kMapItem] = (int)((nn + TPB - 1) / TPB);
-                m.nblk[kMapWarp] = (int)((nn * 32 + TPB - 1) / TPB);
-                m.nblk[kMapWide] = (int)((nn * nn + (long long)TPB * kWideItems - 1) / ((long long)TPB * kWideItems));
-                for (int q = 0; q < 3; ++q) {
-                    m.blk0[q] = blk[q];
-                    blk[q] += m.nblk[q];
-                }
+                m.sec = x; m.a = a; m.b = std::min(a + 2 * s, n); m.mid = std::min(a + s, m.b);
+                const int nn = m.b - m.a;
+                m.blk0 = blk;
+                m.nblk = (nn + TPB / 32 - 1) / (TPB / 32);
+                blk += m.nblk;
                 ms.push_back(m);
+                if (m.mid == m.b) continue;
+                widest = std::max(widest, nn);
+                // rows of each child: its block times its rows of the rank-one eigenvectors; the
+                // number of columns stays on the device (I[9n + a], k_dc_prep)
+                double* W = wsd + secs[x].w_off;
+                const long long sq = (long long)n * n;
+                int* I = wsi + secs[x].i_off;
+                for (int c = 0; c < 2; ++c) {
+                    const int r0 = c == 0 ? m.a : m.mid, r1 = c == 0 ? m.mid : m.b;
+                    GemmProblem P;
+                    std::memset(&P, 0, sizeof(P));
+                    P.M = r1 - r0; P.N = nn; P.K = r1 - r0; P.alpha = 1.0; P.beta = 0.0;
+                    P.dyn_n = I + 9LL * n + m.a;
+                    P.A = W + z_in * sq + r0 + (long long)r0 * n; P.a_si = 1; P.a_sk = n;
+                    P.B = W + sq + r0 + (long long)m.a * n; P.b_sk = 1; P.b_sj = n;
+                    P.C = W + z_out * sq + r0 + (long long)m.a * n; P.c_si = 1; P.c_sj = n; P.c_ji = I + 4LL * n + m.a;
+                    probs.push_back(P);
+                }
             }
         }
-        if (ms.empty()) continue;
         const int nm = (int)ms.size();
         NRG_TRY(bmrg.ensure(sizeof(Merge) * nm));
         NRG_TRY(h2d_async(ctx, bmrg.p, ms.data(), sizeof(Merge) * nm));
         const Merge* dms = bmrg.as<Merge>();
-        k_dc_prep<<<nm, 512, 0, st>>>(dsec, dms, d_V, wsd, wsi);
-        for (int ph = 1; ph <= 4; ++ph)
-            k_dc_phase<<<blk[ph <= 3 ? kMapWarp : kMapItem], TPB, 0, st>>>(dsec, dms, nm, ph, d_V, wsd, wsi,
-                                                                           ctx->d_status.as<int>());
-        k_dc_poscols<<<blk[kMapItem], TPB, 0, st>>>(dsec, dms, nm, d_V, wsd, wsi);
-        ctx->launches += 6;
+        int* d_status = ctx->d_status.as<int>();
+        const size_t psm = std::min(kPrepSmem, 4 * sizeof(double) * (size_t)widest);
+        k_dc_prep<<<nm, kPrepThreads, psm, st>>>(dsec, dms, z_in, d_V, wsd, wsi);
+        k_dc_items<1><<<blk, TPB, 0, st>>>(dsec, dms, nm, z_in, z_out, d_V, wsd, wsi, d_status);
+        k_dc_items<2><<<blk, TPB, 0, st>>>(dsec, dms, nm, z_in, z_out, d_V, wsd, wsi, d_status);
+        k_dc_items<3><<<blk, TPB, 0, st>>>(dsec, dms, nm, z_in, z_out, d_V, wsd, wsi, d_status);
+        ctx->launches += 4;
         NRG_CUDA_TRY(cudaGetLastError());
-        // the number K of non-deflated roots of each merge stays on the device: the
-        // GEMM is launched for K = nn and reads the true K (I[7n + a]) itself
-        std::vector<GemmProblem> probs;
-        for (int i = 0; i < nm; ++i) {
-            const Merge& m = ms[i];
-            const int n = secs[m.sec].n, nn = m.b - m.a;
-            double* W = wsd + secs[m.sec].w_off;
-            const long long sq = (long long)n * n;
-            int* I = wsi + secs[m.sec].i_off;
-            GemmProblem P;
-            std::memset(&P, 0, sizeof(P));
-            P.M = nn; P.N = nn; P.K = nn; P.alpha = 1.0; P.beta = 0.0;
-            P.dyn_nk = I + 7LL * n + m.a;
-            P.A = W + m.a; P.a_si = 1; P.a_sk = n; P.a_ki = I + 5LL * n + m.a;          // Z(:, a+perm[nd[q]])
-            P.B = W + sq + m.a + (long long)m.a * n; P.b_sk = 1; P.b_sj = n;           // U block
-            P.C = W + 2 * sq + m.a; P.c_si = 1; P.c_sj = n; P.c_ji = I + 6LL * n + m.a;  // Qt(:, a+pos[j])
-            probs.push_back(P);
-        }
         NRG_TRY(launch_ggemm(ctx, probs, gslot));
-        k_dc_phase<<<blk[kMapWide], TPB, 0, st>>>(dsec, dms, nm, 5, d_V, wsd, wsi, ctx->d_status.as<int>());
-        k_dc_phase<<<blk[kMapWide], TPB, 0, st>>>(dsec, dms, nm, 6, d_V, wsd, wsi, ctx->d_status.as<int>());
-        ctx->launches += 2;
-        NRG_CUDA_TRY(cudaGetLastError());
+        std::swap(z_in, z_out);
     }
 
     k_large_evals<<<ns, TPB, 0, st>>>(dsec, d_V, d_E, wsd, wsi);
@@ -839,7 +1067,14 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
             return NRG_OK;
         }
     }
-    // otherwise panels of NBB reflectors on grouped GEMMs, last panel first
+    // otherwise panels of NBB reflectors on grouped GEMMs, last panel first, on Z (Qt is their
+    // workspace)
+    for (int x = 0; x < ns; ++x)
+        if (secs[x].z_sel != 0) {
+            double* W = wsd + secs[x].w_off;
+            const size_t sq = (size_t)secs[x].n * secs[x].n;
+            NRG_CUDA_TRY(cudaMemcpyAsync(W, W + 2 * sq, sizeof(double) * sq, cudaMemcpyDeviceToDevice, st));
+        }
     const int qmax = (maxn - 2) / NBB;   // panels cover reflectors 0 .. n-2
     const size_t tf_smem = sizeof(double) * 2 * NBB * NBB;
     NRG_TRY(raise_smem_limit((const void*)k_bt_tfactor, tf_smem));

@@ -121,10 +121,8 @@ __global__ void __launch_bounds__(32 * WM * WN) k_ggemm(const GemmProblem* __res
     const int t = bid - tilePrefix[lo];
     const int tilesN = (P.N + T::TN - 1) / T::TN;
     const int i0 = (t / tilesN) * T::TM, j0 = (t % tilesN) * T::TN;
-    if (P.dyn_nk) {
-        const int v = *P.dyn_nk;
-        P.N = min(P.N, v);
-        P.K = v;
+    if (P.dyn_n) {
+        P.N = min(P.N, *P.dyn_n);
         if (j0 >= P.N) return;
     }
     const bool a_kfast = (P.a_sk == 1 && P.a_si != 1);

@@ -262,9 +262,9 @@ struct GemmProblem {
     const double* B; long long b_sk, b_sj; const int* b_ki; const int* b_ji;
     // C(i,j) = C[ri(i)*c_si + ji(j)*c_sj]
     double* C; long long c_si, c_sj; const int* c_ri; const int* c_ji;
-    // when set, N and K are read from device memory (N = min(N, *dyn_nk), K = *dyn_nk);
-    // the launch is sized for the static N
-    const int* dyn_nk;
+    // when set, N is read from device memory (N = min(N, *dyn_n)); the launch is sized for
+    // the static N
+    const int* dyn_n;
 };
 int launch_ggemm(nrg_context* ctx, std::vector<GemmProblem>& probs, int scratch_slot);
 
