@@ -316,8 +316,8 @@ struct SpikeProb {
     long long s_off, y_off;   // S, Y (kk x nl) col-major in the workspace (y_off < 0: T=0)
     long long ek_off, el_off; // offsets into the energy array (k states, l states)
     int kk, nl, m, toPos, lstride;  // lstride: 1 for consecutive l energies, 0 for a fixed one
-    double sgn, cE, scale, invpf;
-    // full-density-matrix mode: spikes of the sign of this job's bins only; weights
+    double sgn, cE, scale, invpf;   // toPos 1, 0: positive, negative bins; 2: both, by the spike's sign
+    // full-density-matrix mode: each spike in the bins of its sign only; weights
     // P (same offsets as the energies) on both sides; k_is_y: k holds the extra particle
     int fdm, k_is_y;
 };

@@ -165,6 +165,8 @@ __global__ void k_im_gather(const ImGatherProb* __restrict__ probs, const long l
 // One block per tile of 32 k x 64 l spikes of one problem: the tile's bins are first
 // accumulated in a shared-memory window (when they span at most kSpkWin bins), then
 // added to the global bins once per touched bin; the raw sum takes one add per block.
+// A job that feeds both signs' bins (full density matrix) reads its products and takes its
+// logarithms once for the two.
 constexpr int kSpkTK = 32, kSpkTL = 64, kSpkWin = 4096;
 
 __global__ void __launch_bounds__(256) k_spikes(const SpikeProb* __restrict__ probs,
@@ -189,88 +191,103 @@ __global__ void __launch_bounds__(256) k_spikes(const SpikeProb* __restrict__ pr
     const int k1 = tk * kSpkTK + lane;
     const int lb = tl * kSpkTL + warp;
     const double ek = k1 < pr.kk ? E[pr.ek_off + k1] : 0.0;
-    int ia[8], ib[8];
-    double wa[8], wv[8];
-    double wsum = 0.0;
-    int bmin = 0x7fffffff, bmax = -1;
+    // first bin of each spike (0: none), whether it is split with the next one, the share of
+    // the next one, and the weight in the bins of either sign
+    int ia[8];
+    bool split[8];
+    double wb[8], w[2][8];
+    bool ordered = true;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
         const int l = lb + 8 * u;
-        ia[u] = -1;
-        ib[u] = -1;
-        wa[u] = 0.0;
-        wv[u] = 0.0;
+        ia[u] = 0;
+        split[u] = false;
+        wb[u] = w[0][u] = w[1][u] = 0.0;
         if (k1 < pr.kk && l < pr.nl) {
             const long long loc = (long long)k1 + (long long)l * pr.kk;
             const double sv = W[pr.s_off + loc];
             const double el = E[pr.el_off + (long long)l * pr.lstride];
             const double en = pr.sgn * ((ek - pr.cE * el) * pr.scale);
-            double w;
+            const double sy = pr.y_off >= 0 ? sv * W[pr.y_off + loc] : 0.0;
             if (!pr.fdm) {
-                w = (pr.y_off >= 0) ? sv * W[pr.y_off + loc] : sv * sv * pr.invpf;
+                w[0][u] = w[1][u] = (pr.y_off >= 0) ? sy : sv * sv * pr.invpf;
             } else {
                 // both terms of a pair sit at omega = en: the term of the state that gains
                 // the particle (x) enters the positive bins for omega >= 0, the term of the
                 // state that loses it (y) for omega > 0; the rest goes to the negative bins
-                const bool inx = pr.toPos ? (en >= 0.0) : (en < 0.0);
-                const bool iny = pr.toPos ? (en > 0.0) : (en <= 0.0);
                 const double pk = Pw[pr.ek_off + k1], pl = Pw[pr.el_off + (long long)l * pr.lstride];
                 const double px = pr.k_is_y ? pl : pk, py = pr.k_is_y ? pk : pl;
-                w = sv * sv * ((inx ? px : 0.0) + (iny ? py : 0.0));
-                if (pr.y_off >= 0 && (pr.k_is_y ? iny : inx)) w += sv * W[pr.y_off + loc];
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const bool inx = t ? (en >= 0.0) : (en < 0.0);
+                    const bool iny = t ? (en > 0.0) : (en <= 0.0);
+                    w[t][u] = sv * sv * ((inx ? px : 0.0) + (iny ? py : 0.0));
+                    if (pr.y_off >= 0 && (pr.k_is_y ? iny : inx)) w[t][u] += sy;
+                }
             }
-            wsum += w;
             // binningSpike
             const double position = (log10(fabs(en)) - (-15.0)) * 1000.0 + 1.0;
+            ordered = ordered && position == position;
             long long pref = (long long)position;   // int(): truncation toward zero
-            int i1 = 0;
-            if (position <= 0.0) i1 = 1;
-            else if (position >= (double)nbin) i1 = nbin;
             if (pref <= 0) pref = 1;
-            if (i1 > 0) {
-                ia[u] = i1;
-                wa[u] = w;
+            if (position <= 0.0) {
+                ia[u] = 1;
+            } else if (position >= (double)nbin) {
+                ia[u] = nbin;
             } else {
-                const double wb = position - (double)pref;
                 ia[u] = (int)pref;
-                wa[u] = w * (1.0 - wb);
-                ib[u] = (int)pref + 1;
-                wv[u] = w * wb;
+                split[u] = true;
+                wb[u] = position - (double)pref;
             }
-            bmin = min(bmin, ia[u]);
-            bmax = max(bmax, ib[u] >= 0 ? ib[u] : ia[u]);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-        bmin = min(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
-        bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
-    }
-    if (lane == 0) { rs[warp] = wsum; rmin[warp] = bmin; rmax[warp] = bmax; }
-    __syncthreads();
-    double ws = 0.0;
-    int wmin = 0x7fffffff, wmax = -1;
-    for (int q = 0; q < 8; ++q) { ws += rs[q]; wmin = min(wmin, rmin[q]); wmax = max(wmax, rmax[q]); }
-    if (tid == 0 && wmax >= 0) atomicAdd(&tot[2 * pr.m + (pr.toPos ? 1 : 0)], ws);
-    if (wmax < 0) return;
-    double* cont = (pr.toPos ? binPos : binNeg) + ((size_t)pr.m * nbin - 1);
-    const int win = wmax - wmin + 1;
-    if (win <= kSpkWin) {
-        for (int i = tid; i < win; i += 256) hist[i] = 0.0;
-        __syncthreads();
+    // the bins of each sign that the job feeds.  A weight of zero adds nothing to its bins and
+    // does not widen the window, unless its position is not a number.
+    for (int t = pr.toPos == 1 ? 1 : 0; t < (pr.toPos == 0 ? 1 : 2); ++t) {
+        double wsum = 0.0;
+        int bmin = 0x7fffffff, bmax = -1;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            if (ia[u] >= 0) atomicAdd(&hist[ia[u] - wmin], wa[u]);
-            if (ib[u] >= 0) atomicAdd(&hist[ib[u] - wmin], wv[u]);
+            const double wu = t ? w[1][u] : w[0][u];
+            wsum += wu;
+            if (ia[u] > 0 && (wu != 0.0 || !ordered)) {
+                bmin = min(bmin, ia[u]);
+                bmax = max(bmax, ia[u] + (split[u] ? 1 : 0));
+            }
         }
+        for (int o = 16; o > 0; o >>= 1) {
+            wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+            bmin = min(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
+            bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
+        }
+        __syncthreads();   // the previous sign's window has been read
+        if (lane == 0) { rs[warp] = wsum; rmin[warp] = bmin; rmax[warp] = bmax; }
         __syncthreads();
-        for (int i = tid; i < win; i += 256)
-            if (hist[i] != 0.0) atomicAdd(&cont[wmin + i], hist[i]);
-    } else {
+        double ws = 0.0;
+        int wmin = 0x7fffffff, wmax = -1;
+        for (int q = 0; q < 8; ++q) { ws += rs[q]; wmin = min(wmin, rmin[q]); wmax = max(wmax, rmax[q]); }
+        if (wmax < 0) continue;
+        if (tid == 0) atomicAdd(&tot[2 * pr.m + t], ws);
+        double* cont = (t ? binPos : binNeg) + ((size_t)pr.m * nbin - 1);
+        const int win = wmax - wmin + 1;
+        const bool local = win <= kSpkWin;
+        if (local) {
+            for (int i = tid; i < win; i += 256) hist[i] = 0.0;
+            __syncthreads();
+        }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            if (ia[u] >= 0) atomicAdd(&cont[ia[u]], wa[u]);
-            if (ib[u] >= 0) atomicAdd(&cont[ib[u]], wv[u]);
+            const double wu = t ? w[1][u] : w[0][u];
+            if (ia[u] > 0 && (wu != 0.0 || !ordered)) {
+                double* at = local ? &hist[ia[u] - wmin] : &cont[ia[u]];
+                atomicAdd(at, split[u] ? wu * (1.0 - wb[u]) : wu);
+                if (split[u]) atomicAdd(at + 1, wu * wb[u]);
+            }
+        }
+        if (local) {
+            __syncthreads();
+            for (int i = tid; i < win; i += 256)
+                if (hist[i] != 0.0) atomicAdd(&cont[wmin + i], hist[i]);
         }
     }
 }
