@@ -1,4 +1,5 @@
-// FP64 tensor-core MMA (mma.sync m8n8k4 f64) for the products inside the eigensolver's blocks.
+// FP64 tensor-core MMA (mma.sync m8n8k4 f64) and 8-byte asynchronous copies for the products in
+// shared memory.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -11,5 +12,14 @@ __device__ __forceinline__ void cta_dmma(double& d0, double& d1, double a, doubl
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
 }
+
+// 8-byte asynchronous global-to-shared copies (zero-filled when bytes is 0)
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, int bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 }  // namespace nrg

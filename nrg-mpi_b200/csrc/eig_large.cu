@@ -658,15 +658,6 @@ __global__ void __launch_bounds__(256) k_bt_prep(const LSec* __restrict__ secs, 
     for (int e = tid; e < NBB * NBB; e += 256) Tq[e] = Ts[e];
 }
 
-// 8-byte asynchronous global-to-shared copies (zero-filled when bytes is 0)
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, int bytes) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 // Z(:, c0 .. c0+CBK-1) <- H_0 ... H_{n-2} Z(:, ...) panel by panel (last panel first), the
 // column block resident in shared memory; the result goes to the output
 template <int CBK>
@@ -714,17 +705,17 @@ __global__ void __launch_bounds__(256, 1) k_bt_apply(const LSec* __restrict__ se
         const int mr = n - 1 - q * NBB, C = chunks(q);
         if (t == C) {
             const double* Tq = L.R + (size_t)q * NBB * NBB;
-            for (int e = tid; e < NBB * NBB; e += 256) cp_async8(dst + (e % NBB) + (e / NBB) * VLD, Tq + e, 8);
+            for (int e = tid; e < NBB * NBB; e += 256) nrg::cp_async8(dst + (e % NBB) + (e / NBB) * VLD, Tq + e, 8);
         } else {
             const int i0 = 64 * (t < C ? t : t - C - 1), rows = min(64, mr - i0);
             const double* Rp = L.R + bt_panel_off(n, q);
             for (int e = tid; e < 64 * NBB; e += 256) {
                 const int r = e & 63, c = e >> 6;
                 const int rr = r < rows ? r : rows - 1;   // in bounds; nothing is read when zero-filled
-                cp_async8(dst + c * VLD + r, Rp + (size_t)(i0 + rr) + (size_t)c * mr, r < rows ? 8 : 0);
+                nrg::cp_async8(dst + c * VLD + r, Rp + (size_t)(i0 + rr) + (size_t)c * mr, r < rows ? 8 : 0);
             }
         }
-        cp_async_commit();
+        nrg::cp_async_commit();
     };
     int buf = 0;
     issue(qmax, 0, Vb);
@@ -739,8 +730,8 @@ __global__ void __launch_bounds__(256, 1) k_bt_apply(const LSec* __restrict__ se
             double* nxt = Vb + (buf ^ 1) * BUF;
             if (t < 2 * C) issue(q, t + 1, nxt);
             else if (q > 0) issue(q - 1, 0, nxt);
-            if (t < 2 * C || q > 0) cp_async_wait<1>();
-            else cp_async_wait<0>();
+            if (t < 2 * C || q > 0) nrg::cp_async_wait<1>();
+            else nrg::cp_async_wait<0>();
             __syncthreads();
             const double* Vs = Vb + buf * BUF;
             if (t < C) {

@@ -10,202 +10,267 @@
 //   B(k,j) = B[ki(k)*b_sk + ji(j)*b_sj]          ki = b_ki ? b_ki[k] : k, ji likewise
 //   C(i,j) = C[ci(i)*c_si + cj(j)*c_sj]          ci = c_ri ? c_ri[i] : i, cj likewise
 //
-// Output tiles of 32x32 per warp (64x64 with four warps, 32x32 with one, 128x64 and
-// 64x128 with eight), FP64 tensor-core MMA (mma.sync m8n8k4 f64); k slabs of 16 staged in
-// shared memory, the next slab's global loads held in registers while the current slab is
-// multiplied.  Loads are coalesced along whichever index of each operand has unit stride.
+// A problem may be followed by further products of the same C (cont): they are summed in the
+// accumulators of its tiles, one after another, and C is written once.
+//
+// FP64 tensor-core MMA (mma.sync m16n8k8 f64), k in slabs of 32 (16 on the larger tiles) that 8-byte
+// asynchronous copies stage two ahead (every operand is only 8-byte aligned: odd leading dimensions, gathered
+// rows).  Loads are coalesced along whichever index of each operand has unit stride, and a
+// slab is laid out along that index.
 // The tile shape of each launch is chosen by the context's tuner (GemmTuner below).
+#include "cta_gemm.cuh"
 #include "internal.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 namespace nrg {
 namespace {
 
-constexpr int TK = 16;
-
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
+// d (16 x 8) += a (16 x 8) b (8 x 8): lane l holds a(l / 4 + {0, 8}, l % 4 + {0, 4}), b(l % 4 + {0, 4},
+// l / 4) and d(l / 4 + {0, 8}, 2 (l % 4) + {0, 1}); 3-5% over twice m8n8k4 pairs
+__device__ __forceinline__ void dmma16(double (&d)[2][2], const double (&a)[2][2], const double (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%0, %1, %2, %3};\n"
+        : "+d"(d[0][0]), "+d"(d[0][1]), "+d"(d[1][0]), "+d"(d[1][1])
+        : "d"(a[0][0]), "d"(a[1][0]), "d"(a[0][1]), "d"(a[1][1]), "d"(b[0]), "d"(b[1]));
 }
 
-// WM x WN warps per block, each computing a 32 x 32 piece of the (32 WM) x (32 WN) output
-// tile.  Every variant accumulates each output element over k in the same order (slabs of
-// 16, then the k = 4 steps of the MMA), so all variants give bit-identical results and the
-// tile choice is free to change between launches.
-template <int WM, int WN>
+// (16 WM RM) x (8 WN RN) output tile of WM x WN warps with RM x RN MMA tiles each.  Every variant
+// accumulates each output element over k in the same order (the k = 8 steps of the MMA), so all
+// variants give bit-identical results and the tile choice is free to change between launches.
+//
+// What bounds it is the FP64 tensor rate (36 TFLOP/s): registers are kept to 128 so that two
+// blocks of eight warps share an SM and one computes while the other waits for its slab.
+// 64 products of 320 x 320 x 1310 run at 24.4 TFLOP/s on the 64 x 64 tile (slabs of 16: 20.4, of
+// 32: 22.9, with the 16 x 8 x 8 MMA the rest), one of order 4096 at 28.3.  With the slabs staged
+// through registers and 220-255 of them per thread, the products of a shell of N_keep = 4096
+// ran at 8-11 TFLOP/s; 12-20 now, the sectors' ragged sizes taking the rest.
+template <int WM_, int WN_, int RM_, int RN_, int TK_, int ST_, int BLK_>
 struct Tile {
-    static constexpr int TM = 32 * WM, TN = 32 * WN, NT = 32 * WM * WN;
-    static constexpr int LDA = TM + 4, LDB = TN + 4;   // [k][i] and [k][j] rows, padded
-    static constexpr int EA = (TM * TK) / NT, EB = (TN * TK) / NT;
-    static constexpr size_t smem_bytes() { return sizeof(double) * 2 * TK * (LDA + LDB); }
+    static constexpr int WM = WM_, WN = WN_, RM = RM_, RN = RN_;
+    static constexpr int TK = TK_, ST = ST_, BLK = BLK_;   // slab depth, slabs in shared memory, blocks per SM
+    static constexpr int TM = 16 * WM * RM, TN = 8 * WN * RN, NT = 32 * WM * WN;
+    static constexpr int LDK = TK + 4;   // leading dimension of a slab laid out along k
+    static constexpr int SA = TM * LDK, SB = TN * LDK;
+    static constexpr size_t smem_bytes() { return sizeof(double) * ST * (SA + SB); }
+};
+
+// One operand's slabs of TO rows (i of A, j of B) x TK.  A slab whose operand has unit stride
+// along k is stored [row][k] with leading dimension TK + 4, otherwise [k][row] with TO + 4:
+// both 4 mod 16 doubles, so that the copies (16 consecutive) and the MMA fragments (8 rows x 4 k)
+// of a half warp fall on distinct bank pairs.
+template <int TO, int TK, int NT>
+struct Feed {
+    static constexpr int E = TO * TK / NT;   // copies per thread and slab
+    const double* base;
+    const int* ki;
+    long long sk, off[E];
+    int K, k_of, idx[E];
+    unsigned rows;   // copies whose row exists
+    bool kf;
+    __device__ __forceinline__ int row(int u) const {
+        return kf ? (int)threadIdx.x / TK + u * (NT / TK) : (int)threadIdx.x % TO;
+    }
+    __device__ __forceinline__ int col(int u) const {
+        return kf ? (int)threadIdx.x % TK : (int)threadIdx.x / TO + u * (NT / TO);
+    }
+    __device__ __forceinline__ void open(const double* p, long long so, long long sk_, const int* oi, const int* ki_,
+                                         int o0, int extent, int K_) {
+        base = p;
+        ki = ki_;
+        sk = sk_;
+        K = K_;
+        kf = sk_ == 1 && so != 1;
+        rows = 0;
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const int o = o0 + row(u);
+            off[u] = 0;
+            if (o < extent) {
+                off[u] = (oi ? (long long)oi[o] : (long long)o) * so;
+                rows |= 1u << u;
+            }
+            if (!kf) {   // one row per thread
+                rows = o < extent ? ~0u : 0u;
+                break;
+            }
+        }
+        fetch_idx(0);
+    }
+    // the gathered k of the slab at k0, loaded one slab before it is used
+    __device__ __forceinline__ void fetch_idx(int k0) {
+        if (!ki) return;
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const int k = k0 + col(u);
+            idx[u] = k < K ? ki[k] : 0;
+            if (kf) break;   // one k per thread
+        }
+    }
+    __device__ __forceinline__ void issue(double* slab, int k0) {
+        if (kf) {
+            const int k = k0 + col(0);
+            const long long ko = (ki ? idx[0] : k) * sk;
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                const bool in = k < K && (rows >> u & 1u);
+                nrg::cp_async8(slab + row(u) * (TK + 4) + col(u), in ? base + off[u] + ko : base, in ? 8 : 0);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                const int k = k0 + col(u);
+                const bool in = k < K && rows;
+                const long long ko = (ki ? idx[u] : k) * sk;
+                nrg::cp_async8(slab + col(u) * (TO + 4) + row(u), in ? base + off[0] + ko : base, in ? 8 : 0);
+            }
+        }
+        fetch_idx(k0 + TK);
+    }
 };
 
 template <class T>
-struct Slab {
-    double a[T::EA], b[T::EB];
-};
-
-template <class T>
-__device__ __forceinline__ void fetch_slab(const GemmProblem& P, int i0, int j0, int k0, Slab<T>& r, bool a_kfast,
-                                           bool b_kfast) {
-    const int tid = threadIdx.x;
-#pragma unroll
-    for (int u = 0; u < T::EA; ++u) {
-        const int e = tid + u * T::NT;
-        int ii, kk;
-        if (a_kfast) { kk = e % TK; ii = e / TK; } else { ii = e % T::TM; kk = e / T::TM; }
-        const int gi = i0 + ii, gk = k0 + kk;
-        double v = 0.0;
-        if (gi < P.M && gk < P.K) {
-            const long long ri = P.a_ri ? P.a_ri[gi] : gi;
-            const long long ki = P.a_ki ? P.a_ki[gk] : gk;
-            v = P.A[ri * P.a_si + ki * P.a_sk];
-        }
-        r.a[u] = v;
-    }
-#pragma unroll
-    for (int u = 0; u < T::EB; ++u) {
-        const int e = tid + u * T::NT;
-        int jj, kk;
-        if (b_kfast) { kk = e % TK; jj = e / TK; } else { jj = e % T::TN; kk = e / T::TN; }
-        const int gj = j0 + jj, gk = k0 + kk;
-        double v = 0.0;
-        if (gj < P.N && gk < P.K) {
-            const long long ki = P.b_ki ? P.b_ki[gk] : gk;
-            const long long ji = P.b_ji ? P.b_ji[gj] : gj;
-            v = P.B[ki * P.b_sk + ji * P.b_sj];
-        }
-        r.b[u] = v;
-    }
-}
-
-template <class T>
-__device__ __forceinline__ void store_slab(const Slab<T>& r, double* As, double* Bs, bool a_kfast, bool b_kfast) {
-    const int tid = threadIdx.x;
-#pragma unroll
-    for (int u = 0; u < T::EA; ++u) {
-        const int e = tid + u * T::NT;
-        int ii, kk;
-        if (a_kfast) { kk = e % TK; ii = e / TK; } else { ii = e % T::TM; kk = e / T::TM; }
-        As[kk * T::LDA + ii] = r.a[u];
-    }
-#pragma unroll
-    for (int u = 0; u < T::EB; ++u) {
-        const int e = tid + u * T::NT;
-        int jj, kk;
-        if (b_kfast) { kk = e % TK; jj = e / TK; } else { jj = e % T::TN; kk = e / T::TN; }
-        Bs[kk * T::LDB + jj] = r.b[u];
-    }
-}
-
-template <int WM, int WN>
-__global__ void __launch_bounds__(32 * WM * WN) k_ggemm(const GemmProblem* __restrict__ probs,
-                                                        const int* __restrict__ tilePrefix, int nprob) {
-    using T = Tile<WM, WN>;
+__global__ void __launch_bounds__(T::NT, T::BLK) k_ggemm(const GemmProblem* __restrict__ probs,
+                                                    const int* __restrict__ tilePrefix, int nprob) {
     extern __shared__ double gsm[];
-    // two A slabs, then two B slabs
-    auto As = [&](int x) { return gsm + x * (TK * T::LDA); };
-    auto Bs = [&](int x) { return gsm + 2 * TK * T::LDA + x * (TK * T::LDB); };
     const int bid = blockIdx.x;
     int lo = 0, hi = nprob - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (tilePrefix[mid] <= bid) lo = mid; else hi = mid - 1;
     }
-    GemmProblem P = probs[lo];
+    const GemmProblem& P = probs[lo];
     const int t = bid - tilePrefix[lo];
     const int tilesN = (P.N + T::TN - 1) / T::TN;
     const int i0 = (t / tilesN) * T::TM, j0 = (t % tilesN) * T::TN;
-    if (P.dyn_n) {
-        P.N = min(P.N, *P.dyn_n);
-        if (j0 >= P.N) return;
-    }
-    const bool a_kfast = (P.a_sk == 1 && P.a_si != 1);
-    const bool b_kfast = (P.b_sk == 1 && P.b_sj != 1);
+    const int M = P.M, N = P.dyn_n ? min(P.N, *P.dyn_n) : P.N;
+    if (j0 >= N) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wi = (warp / WN) * 32, wj = (warp % WN) * 32;   // warp tile origin
+    const int wi = (warp % T::WM) * 16 * T::RM, wj = (warp / T::WM) * 8 * T::RN;   // warp tile origin
     const int g = lane >> 2, q4 = lane & 3;
-    double acc[4][4][2];
+    // MMA tiles of the warp that hold any output: a tile at the edge leaves the tensor pipe to the
+    // others (order 333 on 64 x 64: 27 tiles' work instead of 36)
+    const int rl = min(T::RM, max(0, (M - i0 - wi + 15) / 16)), cl = min(T::RN, max(0, (N - j0 - wj + 7) / 8));
+    double acc[T::RM][T::RN][2][2];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < T::RM; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c][0] = acc[r][c][1] = 0.0;
-    const int nslab = (P.K + TK - 1) / TK;
-    Slab<T> reg;
-    if (nslab > 0) {
-        fetch_slab<T>(P, i0, j0, 0, reg, a_kfast, b_kfast);
-        store_slab<T>(reg, As(0), Bs(0), a_kfast, b_kfast);
-    }
-    __syncthreads();
-    for (int s = 0; s < nslab; ++s) {
-        const int cur = s & 1;
-        if (s + 1 < nslab) fetch_slab<T>(P, i0, j0, (s + 1) * TK, reg, a_kfast, b_kfast);
-        const double* as = As(cur);
-        const double* bs = Bs(cur);
+        for (int c = 0; c < T::RN; ++c)
+            acc[r][c][0][0] = acc[r][c][0][1] = acc[r][c][1][0] = acc[r][c][1][1] = 0.0;
+    // the problem's slabs, then those of the problems added to it
+    for (int x = lo; x == lo || (x < nprob && probs[x].cont); ++x) {
+        const GemmProblem& Q = probs[x];
+        Feed<T::TM, T::TK, T::NT> fa;
+        Feed<T::TN, T::TK, T::NT> fb;
+        fa.open(Q.A, Q.a_si, Q.a_sk, Q.a_ri, Q.a_ki, i0, M, Q.K);
+        fb.open(Q.B, Q.b_sj, Q.b_sk, Q.b_ji, Q.b_ki, j0, N, Q.K);
+        const int nslab = (Q.K + T::TK - 1) / T::TK;
+        // strides of the fragments in a slab
+        const int ai = fa.kf ? T::LDK : 1, ak = fa.kf ? 1 : T::TM + 4;
+        const int bj = fb.kf ? T::LDK : 1, bk = fb.kf ? 1 : T::TN + 4;
+        const int a_at = (wi + g) * ai + q4 * ak, b_at = (wj + g) * bj + q4 * bk;
 #pragma unroll
-        for (int ks = 0; ks < TK; ks += 4) {
-            double af[4], bf[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) af[r] = as[(ks + q4) * T::LDA + wi + r * 8 + g];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) bf[c] = bs[(ks + q4) * T::LDB + wj + c * 8 + g];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) dmma(acc[r][c][0], acc[r][c][1], af[r], bf[c]);
+        for (int s = 0; s < T::ST - 1; ++s) {
+            if (s < nslab) {
+                fa.issue(gsm + s * T::SA, s * T::TK);
+                fb.issue(gsm + T::ST * T::SA + s * T::SB, s * T::TK);
+            }
+            nrg::cp_async_commit();
         }
-        if (s + 1 < nslab) store_slab<T>(reg, As(cur ^ 1), Bs(cur ^ 1), a_kfast, b_kfast);
-        __syncthreads();
+        int cur = 0, ahead = T::ST - 1;
+        for (int s = 0; s < nslab; ++s) {
+            nrg::cp_async_wait<T::ST - 2>();
+            __syncthreads();   // slab s has landed; every warp is through with slab s - 1
+            if (s + T::ST - 1 < nslab) {
+                fa.issue(gsm + ahead * T::SA, (s + T::ST - 1) * T::TK);
+                fb.issue(gsm + T::ST * T::SA + ahead * T::SB, (s + T::ST - 1) * T::TK);
+            }
+            nrg::cp_async_commit();
+            const double* as = gsm + cur * T::SA + a_at;
+            const double* bs = gsm + T::ST * T::SA + cur * T::SB + b_at;
+            auto multiply = [&](auto whole) {
+#pragma unroll
+                for (int ks = 0; ks < T::TK; ks += 8) {
+                    double af[T::RM][2][2], bf[T::RN][2];
+#pragma unroll
+                    for (int r = 0; r < T::RM; ++r)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            af[r][h][0] = as[ks * ak + (16 * r + 8 * h) * ai];
+                            af[r][h][1] = as[(ks + 4) * ak + (16 * r + 8 * h) * ai];
+                        }
+#pragma unroll
+                    for (int c = 0; c < T::RN; ++c) {
+                        bf[c][0] = bs[ks * bk + c * 8 * bj];
+                        bf[c][1] = bs[(ks + 4) * bk + c * 8 * bj];
+                    }
+#pragma unroll
+                    for (int r = 0; r < T::RM; ++r)
+#pragma unroll
+                        for (int c = 0; c < T::RN; ++c)
+                            if (decltype(whole)::value || (r < rl && c < cl)) dmma16(acc[r][c], af[r], bf[c]);
+                }
+            };
+            // (two copies of the loop are only worth their registers on the small warp tiles)
+            if (T::RM * T::RN > 4 ? rl > 0 && cl > 0 : rl == T::RM && cl == T::RN) multiply(std::true_type());
+            else if (T::RM * T::RN <= 4 && rl > 0 && cl > 0) multiply(std::false_type());
+            ahead = cur;
+            cur = cur + 1 == T::ST ? 0 : cur + 1;
+        }
+        nrg::cp_async_wait<0>();
+        __syncthreads();   // the slabs may be overwritten
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < 2 * T::RM; ++r) {
         const int gi = i0 + wi + r * 8 + g;
-        if (gi >= P.M) continue;
+        if (gi >= M) continue;
         const long long ci = P.c_ri ? P.c_ri[gi] : gi;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < T::RN; ++c) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int gj = j0 + wj + c * 8 + 2 * q4 + h;
-                if (gj >= P.N) continue;
+                if (gj >= N) continue;
                 const long long cj = P.c_ji ? P.c_ji[gj] : gj;
                 double* out = P.C + ci * P.c_si + cj * P.c_sj;
-                const double v = P.alpha * acc[r][c][h];
+                const double v = P.alpha * acc[r / 2][c][r % 2][h];
                 *out = (P.beta == 0.0) ? v : P.beta * *out + v;
             }
         }
     }
 }
 
-// the tile variants, in the order of GemmTuner's slots
-constexpr int kVariants = 4;
-constexpr int kWM[kVariants] = {2, 1, 4, 2};
-constexpr int kWN[kVariants] = {2, 1, 2, 4};
-
-template <int WM, int WN>
-int launch_variant(nrg_context* ctx, long long total_blocks_hint, const GemmProblem* dp, const int* dq, int np,
-                   const std::vector<GemmProblem>& live, std::vector<int>& prefix, DevBuf& prefixBuf) {
-    using T = Tile<WM, WN>;
+template <class T>
+int launch_variant(nrg_context* ctx, const std::vector<GemmProblem>& live, DevBuf& buf) {
+    const int np = (int)live.size();
+    std::vector<int> prefix(np);
     long long total = 0;
     for (int i = 0; i < np; ++i) {
-        prefix[i] = (int)total;
-        total += (long long)((live[i].M + T::TM - 1) / T::TM) * ((live[i].N + T::TN - 1) / T::TN);
+        prefix[i] = (int)total;   // an added product has no tiles of its own
+        if (!live[i].cont) total += (long long)((live[i].M + T::TM - 1) / T::TM) * ((live[i].N + T::TN - 1) / T::TN);
     }
-    (void)total_blocks_hint;
     if (total > 0x7fffffffLL) return NRG_ERR_TOO_LARGE;
-    NRG_TRY(h2d_async(ctx, prefixBuf.p, prefix.data(), sizeof(int) * np));
-    const size_t smem = T::smem_bytes();
-    if (smem > 48 * 1024) NRG_TRY(raise_smem_limit((const void*)k_ggemm<WM, WN>, smem));
-    k_ggemm<WM, WN><<<(unsigned)total, T::NT, smem, ctx->stream>>>(dp, dq, np);
+    const GemmProblem* dp = nullptr;
+    const int* dq = nullptr;
+    NRG_TRY(h2d_pair(ctx, buf, live, prefix, &dp, &dq));
+    NRG_TRY(raise_smem_limit((const void*)k_ggemm<T>, T::smem_bytes()));
+    k_ggemm<T><<<(unsigned)total, T::NT, T::smem_bytes(), ctx->stream>>>(dp, dq, np);
     ctx->launches++;
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
 }
+
+// the tile variants, in the order of GemmTuner's slots: 64 x 64, 32 x 32, 128 x 64, 64 x 128
+using Tile0 = Tile<2, 4, 2, 2, 32, 3, 2>;
+using Tile1 = Tile<2, 2, 1, 2, 32, 3, 4>;
+using Tile2 = Tile<4, 2, 2, 4, 16, 3, 2>;
+using Tile3 = Tile<2, 4, 2, 4, 16, 3, 2>;
 
 int log2_bucket(long long v) {
     int b = 0;
@@ -274,11 +339,27 @@ GemmTuner& tuner_for(int dev) {
 }
 
 int launch_ggemm(nrg_context* ctx, std::vector<GemmProblem>& probs, int scratch_slot) {
-    // drop empty problems
     std::vector<GemmProblem> live;
     live.reserve(probs.size());
-    for (auto& p : probs)
-        if (p.M > 0 && p.N > 0 && p.K > 0) live.push_back(p);
+    // empty problems dropped, the others by decreasing length of their sums (a tile's time), those added to a product
+    // behind it: a long tile that starts last runs alone
+    std::vector<std::array<long long, 3>> sums;   // -K in total, first problem, end
+    for (size_t x = 0; x < probs.size(); ++x) {
+        if (!probs[x].cont || sums.empty()) sums.push_back({0, (long long)x, 0});
+        if (probs[x].M > 0 && probs[x].N > 0 && probs[x].K > 0) sums.back()[0] -= probs[x].K;
+        sums.back()[2] = (long long)x + 1;
+    }
+    std::stable_sort(sums.begin(), sums.end(), [](const auto& a, const auto& b) { return a[0] < b[0]; });
+    for (const auto& q : sums) {
+        bool added = false;
+        for (long long x = q[1]; x < q[2]; ++x) {
+            const GemmProblem& p = probs[x];
+            if (p.M <= 0 || p.N <= 0 || p.K <= 0) continue;
+            live.push_back(p);
+            live.back().cont = added;
+            added = true;
+        }
+    }
     const int np = (int)live.size();
     if (np == 0) return NRG_OK;
     // problem-mix key and algorithmic flops
@@ -302,13 +383,7 @@ int launch_ggemm(nrg_context* ctx, std::vector<GemmProblem>& probs, int scratch_
     std::unique_lock<std::mutex> lk(tu.mu);
     tu.collect(false);
     const int v = tu.pick(key);
-    DevBuf& dp = ctx->scratch.b[scratch_slot];
-    DevBuf& dq = ctx->scratch.b[scratch_slot + 1];
-    NRG_TRY(dp.ensure(sizeof(GemmProblem) * np));
-    NRG_TRY(dq.ensure(sizeof(int) * np));
-    for (auto& p : live) p.tiles = 0;   // unused by the kernels (the prefix carries the tiling)
-    NRG_TRY(h2d_async(ctx, dp.p, live.data(), sizeof(GemmProblem) * np));
-    std::vector<int> prefix(np);
+    DevBuf& buf = ctx->scratch.b[scratch_slot];
     const bool timed = tu.table[key].samples[v] < GemmTuner::kSamples && tu.table[key].inflight[v] == 0;
     cudaEvent_t ea = nullptr, eb = nullptr;
     if (timed) {
@@ -320,10 +395,10 @@ int launch_ggemm(nrg_context* ctx, std::vector<GemmProblem>& probs, int scratch_
     if (timed) NRG_CUDA_TRY(cudaEventRecord(ea, ctx->stream));
     int rc = NRG_OK;
     switch (v) {
-        case 0: rc = launch_variant<kWM[0], kWN[0]>(ctx, 0, dp.as<GemmProblem>(), dq.as<int>(), np, live, prefix, dq); break;
-        case 1: rc = launch_variant<kWM[1], kWN[1]>(ctx, 0, dp.as<GemmProblem>(), dq.as<int>(), np, live, prefix, dq); break;
-        case 2: rc = launch_variant<kWM[2], kWN[2]>(ctx, 0, dp.as<GemmProblem>(), dq.as<int>(), np, live, prefix, dq); break;
-        default: rc = launch_variant<kWM[3], kWN[3]>(ctx, 0, dp.as<GemmProblem>(), dq.as<int>(), np, live, prefix, dq); break;
+        case 0: rc = launch_variant<Tile0>(ctx, live, buf); break;
+        case 1: rc = launch_variant<Tile1>(ctx, live, buf); break;
+        case 2: rc = launch_variant<Tile2>(ctx, live, buf); break;
+        default: rc = launch_variant<Tile3>(ctx, live, buf); break;
     }
     if (timed) {
         const bool rec = rc == NRG_OK && cudaEventRecord(eb, ctx->stream) == cudaSuccess;

@@ -3,6 +3,7 @@
 #pragma once
 #include "common.cuh"
 
+#include <cstring>
 #include <string>
 #include <vector>
 #include <map>
@@ -251,11 +252,28 @@ int raise_smem_limit(const void* func, size_t bytes);
 // stream-ordered upload of a small host array through the pinned staging ring (the host
 // array may be reused as soon as the call returns)
 int h2d_async(nrg_context* ctx, void* dst, const void* src, size_t bytes);
+// a descriptor list and its prefix in one buffer with one copy
+template <class A, class B>
+int h2d_pair(nrg_context* ctx, DevBuf& buf, const std::vector<A>& a, const std::vector<B>& b, const A** da,
+             const B** db) {
+    static_assert(sizeof(A) % 8 == 0, "the second list starts on an 8-byte boundary");
+    const size_t na = sizeof(A) * a.size(), nb = sizeof(B) * b.size();
+    std::vector<char> both(na + nb);
+    if (na) std::memcpy(both.data(), a.data(), na);
+    if (nb) std::memcpy(both.data() + na, b.data(), nb);
+    NRG_TRY(buf.ensure(na + nb));
+    NRG_TRY(h2d_async(ctx, buf.p, both.data(), na + nb));
+    *da = buf.as<A>();
+    *db = reinterpret_cast<const B*>(buf.as<char>() + na);
+    return NRG_OK;
+}
 
 // ---- grouped gather GEMM -------------------------------------------------------------
 struct GemmProblem {
     int M, N, K;
-    int tiles;              // filled by the launcher
+    // 1: this product is added to the one before it in the list (same M, N, alpha and C), in
+    // the same output tiles; its beta is not read
+    int cont;
     double alpha, beta;
     // A(i,k) = A[ri(i)*a_si + ki(k)*a_sk], ri = a_ri ? a_ri[i] : i, ki = a_ki ? a_ki[k] : k
     const double* A; long long a_si, a_sk; const int* a_ri; const int* a_ki;

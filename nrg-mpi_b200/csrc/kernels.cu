@@ -295,8 +295,10 @@ __global__ void __launch_bounds__(256) k_spikes(const SpikeProb* __restrict__ pr
 // calcThermo (module.F90:1931-1982) on one iteration's eigenvalues in sector order, before
 // truncation (postprocess.F90:62): Z, E = sum bE e^-bE, <Sz^2>, <Sz> with bE = betabar E,
 // then C = sum (bE - E/Z)^2 e^-bE / Z (the fluctuation form), S = E/Z + ln Z and
-// X = <Sz^2> - <Sz>^2.  One block; partial sums per thread, combined in a fixed order.
-// tab: sector start | dimension | 2 Sz, nsub entries each.
+// X = <Sz^2> - <Sz>^2.  One block over the states of all sectors; partial sums per thread,
+// combined in a fixed order.  (Sector after sector, each a round trip to memory, took 69 us at
+// N_keep = 4096; 38 now.)
+// tab: sector start | 2 Sz | states before the sector, nsub entries each, and all states.
 __device__ __forceinline__ void thermo_sum(double* v, int nv, double (*red)[32]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int q = 0; q < nv; ++q)
@@ -311,32 +313,33 @@ __device__ __forceinline__ void thermo_sum(double* v, int nv, double (*red)[32])
         v[q] = s;
     }
 }
-__global__ void __launch_bounds__(512) k_thermo(const double* __restrict__ E, const int* __restrict__ tab,
+__global__ void __launch_bounds__(1024) k_thermo(const double* __restrict__ E, const int* __restrict__ tab,
                                                 int nsub, double betabar, double* __restrict__ out) {
     __shared__ double red[4][32];
     double v[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int s = 0; s < nsub; ++s) {
-        const int s0 = tab[s], d = tab[nsub + s];
-        const double sz = 0.5 * tab[2 * nsub + s];
-        for (int i = threadIdx.x; i < d; i += blockDim.x) {
-            const double bE = betabar * E[s0 + i];
-            const double ex = exp(-bE);
-            v[0] += ex;
-            v[1] += bE * ex;
-            v[2] += ex * sz * sz;
-            v[3] += ex * sz;
+    const int* before = tab + 2 * nsub;   // states before each sector, and in all
+    auto states = [&](auto&& add) {
+        for (int i = threadIdx.x; i < before[nsub]; i += blockDim.x) {
+            int lo = 0, hi = nsub - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (before[mid] <= i) lo = mid; else hi = mid - 1;
+            }
+            add(betabar * E[tab[lo] + (i - before[lo])], lo);
         }
-    }
+    };
+    states([&](double bE, int s) {
+        const double sz = 0.5 * tab[nsub + s];
+        const double ex = exp(-bE);
+        v[0] += ex;
+        v[1] += bE * ex;
+        v[2] += ex * sz * sz;
+        v[3] += ex * sz;
+    });
     thermo_sum(v, 4, red);
     const double Z = v[0], em = v[1] / Z;
     double c[1] = {0.0};
-    for (int s = 0; s < nsub; ++s) {
-        const int s0 = tab[s], d = tab[nsub + s];
-        for (int i = threadIdx.x; i < d; i += blockDim.x) {
-            const double bE = betabar * E[s0 + i];
-            c[0] += (bE - em) * (bE - em) * exp(-bE);
-        }
-    }
+    states([&](double bE, int) { c[0] += (bE - em) * (bE - em) * exp(-bE); });
     thermo_sum(c, 1, red);
     if (threadIdx.x == 0) {
         out[0] = c[0] / Z;
@@ -433,13 +436,16 @@ __global__ void k_sum_bins(const double* bins, int nbin, double* out) {
         out[m] = r;
     }
 }
-// sum of the diagonals of row-major square blocks
+// sum of the diagonals of row-major square blocks: a warp per block at a time, so that the
+// strided loads of many blocks are in flight together (48 blocks: 27 us one after another)
 __global__ void k_trace(const double* rdm, const long long* offs, const int* dims, int nblk, double* out) {
     __shared__ double red[32];
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) {
+    for (int b = threadIdx.x >> 5; b < nblk; b += blockDim.x >> 5) {
         const int n = dims[b];
-        for (int i = threadIdx.x; i < n; i += blockDim.x) s += rdm[offs[b] + (long long)i * n + i];
+        const double* d = rdm + offs[b];
+#pragma unroll 8
+        for (int i = threadIdx.x & 31; i < n; i += 32) s += d[(long long)i * n + i];
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -547,19 +553,15 @@ int run_spikes(nrg_context* ctx, std::vector<SpikeProb>& probs, const double* d_
     }
     if (total == 0) return NRG_OK;
     if (total > 0x7fffffffLL) return NRG_ERR_TOO_LARGE;
-    DevBuf& dp = ctx->scratch.b[18];
-    DevBuf& dq = ctx->scratch.b[19];
-    NRG_TRY(dp.ensure(sizeof(SpikeProb) * np));
-    NRG_TRY(dq.ensure(sizeof(long long) * np));
-    NRG_TRY(h2d_async(ctx, dp.p, probs.data(), sizeof(SpikeProb) * np));
-    NRG_TRY(h2d_async(ctx, dq.p, prefix.data(), sizeof(long long) * np));
+    const SpikeProb* dp = nullptr;
+    const long long* dq = nullptr;
+    NRG_TRY(h2d_pair(ctx, ctx->scratch.b[18], probs, prefix, &dp, &dq));
     for (const auto& p : probs)
         if (p.fdm && !d_P) {
             nrg_set_error_message("full-density-matrix spikes without weights");
             return NRG_ERR_INVALID;
         }
-    k_spikes<<<(unsigned)total, 256, 0, ctx->stream>>>(dp.as<SpikeProb>(), dq.as<long long>(), np, d_work, d_E, nbin,
-                                                     d_binPos, d_binNeg, d_tot, d_P);
+    k_spikes<<<(unsigned)total, 256, 0, ctx->stream>>>(dp, dq, np, d_work, d_E, nbin, d_binPos, d_binNeg, d_tot, d_P);
     ctx->launches++;
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
@@ -568,18 +570,18 @@ int run_spikes(nrg_context* ctx, std::vector<SpikeProb>& probs, const double* d_
 int run_thermo(nrg_context* ctx, const Sectors& S, const double* d_E, double* d_out) {
     const Model& M = ctx->model;
     const int nsub = S.nsub, nVar = S.nVar;
-    std::vector<int> tab(3 * (size_t)nsub);
+    std::vector<int> tab(3 * (size_t)nsub + 1);
     for (int s = 0; s < nsub; ++s) {
         int sz = 0;
         for (int v = M.cb[1]; v <= M.cb[3]; ++v) sz += S.qn[(size_t)s * nVar + v - 1];
         tab[s] = S.start[s];
-        tab[nsub + s] = S.dim[s];
-        tab[2 * nsub + s] = sz;
+        tab[nsub + s] = sz;
+        tab[2 * nsub + s + 1] = tab[2 * nsub + s] + S.dim[s];
     }
     DevBuf& b = ctx->scratch.b[38];
     NRG_TRY(b.ensure(sizeof(int) * tab.size()));
     NRG_TRY(h2d_async(ctx, b.p, tab.data(), sizeof(int) * tab.size()));
-    k_thermo<<<1, 512, 0, ctx->stream>>>(d_E, b.as<int>(), nsub, kBetabar, d_out);
+    k_thermo<<<1, 1024, 0, ctx->stream>>>(d_E, b.as<int>(), nsub, kBetabar, d_out);
     ctx->launches++;
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
@@ -608,15 +610,11 @@ int run_gather_segs(nrg_context* ctx, const double* src, double* dst, long long 
         total += (long long)segs[i].len * segs[i].count;
     }
     if (total == 0) return NRG_OK;
-    DevBuf& bs = ctx->scratch.b[20];
-    DevBuf& bp = ctx->scratch.b[23];
-    NRG_TRY(bs.ensure(sizeof(HostSeg) * ns));
-    NRG_TRY(bp.ensure(sizeof(long long) * ns));
-    NRG_TRY(h2d_async(ctx, bs.p, segs.data(), sizeof(HostSeg) * ns));
-    NRG_TRY(h2d_async(ctx, bp.p, prefix.data(), sizeof(long long) * ns));
+    const HostSeg* ds = nullptr;
+    const long long* dp = nullptr;
+    NRG_TRY(h2d_pair(ctx, ctx->scratch.b[20], segs, prefix, &ds, &dp));
     const long long grid = std::min<long long>((total + 255) / 256, 148LL * 16);
-    k_gather_segs<<<(unsigned)grid, 256, 0, ctx->stream>>>(src, dst, ld, bs.as<HostSeg>(), bp.as<long long>(), ns,
-                                                          total, packed ? 1 : 0);
+    k_gather_segs<<<(unsigned)grid, 256, 0, ctx->stream>>>(src, dst, ld, ds, dp, ns, total, packed ? 1 : 0);
     ctx->launches++;
     NRG_CUDA_TRY(cudaGetLastError());
     *bytes = total * (long long)sizeof(double);
@@ -634,15 +632,11 @@ int run_scaled_gather(nrg_context* ctx, const std::vector<ScaledGather>& jobs, d
         total += (long long)jobs[i].n * jobs[i].nc;
     }
     if (total == 0) return NRG_OK;
-    DevBuf& bj = ctx->scratch.b[40];
-    DevBuf& bp = ctx->scratch.b[41];
-    NRG_TRY(bj.ensure(sizeof(ScaledGather) * nj));
-    NRG_TRY(bp.ensure(sizeof(long long) * nj));
-    NRG_TRY(h2d_async(ctx, bj.p, jobs.data(), sizeof(ScaledGather) * nj));
-    NRG_TRY(h2d_async(ctx, bp.p, prefix.data(), sizeof(long long) * nj));
+    const ScaledGather* dj = nullptr;
+    const long long* dp = nullptr;
+    NRG_TRY(h2d_pair(ctx, ctx->scratch.b[40], jobs, prefix, &dj, &dp));
     const long long grid = std::min<long long>((total + 255) / 256, 148LL * 16);
-    k_scaled_gather<<<(unsigned)grid, 256, 0, ctx->stream>>>(bj.as<ScaledGather>(), bp.as<long long>(), nj, total, dst,
-                                                            V, rows, P);
+    k_scaled_gather<<<(unsigned)grid, 256, 0, ctx->stream>>>(dj, dp, nj, total, dst, V, rows, P);
     ctx->launches++;
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
