@@ -594,13 +594,21 @@ __device__ __forceinline__ long long bt_panel_off(int n, int q) {
 }
 
 // explicit V_q, its Gram matrix and T_q (dlarft, forward, columnwise) for every panel of
-// every sector at once: one block per (panel, sector)
+// every sector at once: one block per (panel, sector).  The Gram matrix is on the FP64 MMA, each
+// warp five 8 x 8 tiles of a row (tiles row + 0 .. 4 modulo 8 hold every pair of columns), the
+// next 64 rows loaded meanwhile.  T is put together from two halves, whose recursions run in
+// one warp each with a row of T per lane, T12 = -T1 G12 T2: the recursion over all 64 columns in
+// shared memory, two barriers a column, was most of the kernel's 0.34 ms for 4 sectors of order
+// 1150 (0.06 ms now).
+constexpr int kPrepLd = NBB + 4;   // 4 mod 16 doubles: conflict-free MMA operands
+constexpr size_t kBtPrepSmem = sizeof(double) * 3 * NBB * kPrepLd;
 __global__ void __launch_bounds__(256) k_bt_prep(const LSec* __restrict__ secs, double* eigbuf, double* wsd,
                                                  int* wsi) {
+    constexpr int LD = kPrepLd, H = NBB / 2, LDX = H + 4;
     extern __shared__ double bsm[];
-    double* Vs = bsm;                  // chunk of the panel, Vs[c * 65 + r]
-    double* G = Vs + NBB * 65;         // NBB x NBB, column-major
-    double* Ts = G + NBB * NBB;        // NBB x NBB, column-major
+    double* Vs = bsm;                  // 64 rows of the panel, Vs[c * LD + r]
+    double* G = Vs + NBB * LD;         // G[i * LD + j], tiles of the upper triangle
+    double* Ts = G + NBB * LD;         // T(p, c) at Ts[c * LD + p]
     const LSec sec = secs[blockIdx.y];
     const int n = sec.n, nr = n - 1, q = blockIdx.x, jb = q * NBB;
     if (jb >= nr) return;
@@ -608,54 +616,92 @@ __global__ void __launch_bounds__(256) k_bt_prep(const LSec* __restrict__ secs, 
     const int b = min(NBB, nr - jb), r0 = jb + 1, mr = n - r0;
     double* Rp = L.R + bt_panel_off(n, q);
     double* Tq = L.R + (size_t)q * NBB * NBB;
-    const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
-    double g[4][4];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q4 = lane & 3;
+    const int r = tid & 63, cb = tid >> 6;   // the thread's row and columns cb + 4 u of a chunk
+    double v[NBB / 4];
+    auto load = [&](int i0) {
+        const int row = r0 + i0 + r;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+        for (int u = 0; u < NBB / 4; ++u) {
+            const int c = cb + 4 * u, k = jb + c;
+            v[u] = 0.0;
+            if (i0 + r < mr && c < b) v[u] = row == k + 1 ? 1.0 : (row > k + 1 ? L.A[(size_t)row + (size_t)k * n] : 0.0);
+        }
+    };
+    double acc[5][2];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) g[a][c] = 0.0;
+    for (int d = 0; d < 5; ++d) acc[d][0] = acc[d][1] = 0.0;
+    load(0);
     for (int i0 = 0; i0 < mr; i0 += 64) {
-        const int rows = min(64, mr - i0);
-        for (int e = tid; e < 64 * NBB; e += 256) {
-            const int r = e & 63, c = e >> 6;
-            const int row = r0 + i0 + r, k = jb + c;
-            double v = 0.0;
-            if (r < rows && c < b) v = (row == k + 1) ? 1.0 : (row > k + 1 ? L.A[(size_t)row + (size_t)k * n] : 0.0);
-            Vs[c * 65 + r] = v;
-            if (r < rows) Rp[(size_t)(i0 + r) + (size_t)c * mr] = v;
+#pragma unroll
+        for (int u = 0; u < NBB / 4; ++u) {
+            const int c = cb + 4 * u;
+            Vs[c * LD + r] = v[u];
+            if (i0 + r < mr) Rp[(size_t)(i0 + r) + (size_t)c * mr] = v[u];
         }
         __syncthreads();
-        for (int r = 0; r < rows; ++r) {
-            double x[4], y[4];
+        if (i0 + 64 < mr) load(i0 + 64);
+#pragma unroll 4
+        for (int k0 = 0; k0 < 64; k0 += 4) {
+            const double a = Vs[(8 * warp + g) * LD + k0 + q4];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                x[a] = Vs[(ti * 4 + a) * 65 + r];
-                y[a] = Vs[(tj * 4 + a) * 65 + r];
-            }
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) g[a][c] = fma(x[a], y[c], g[a][c]);
+            for (int d = 0; d < 5; ++d)
+                nrg::cta_dmma(acc[d][0], acc[d][1], a, Vs[(8 * ((warp + d) & 7) + g) * LD + k0 + q4]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int d = 0; d < 5; ++d)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) G[(ti * 4 + a) + (tj * 4 + c) * NBB] = g[a][c];
-    for (int e = tid; e < NBB * NBB; e += 256) Ts[e] = 0.0;
+        for (int h = 0; h < 2; ++h) {
+            const int i = 8 * warp + g, j = 8 * ((warp + d) & 7) + 2 * q4 + h;
+            if (i <= j) G[i * LD + j] = acc[d][h];
+            if (i > j && d < 4) G[j * LD + i] = acc[d][h];   // d = 4 has its mirror in another warp
+        }
+    for (int e = tid; e < H * H; e += 256) Ts[(e / H) * LD + H + e % H] = 0.0;   // below the diagonal blocks
     __syncthreads();
-    for (int c = 0; c < b; ++c) {
-        const double tc = L.TAU[jb + c];
-        double acc = 0.0;
-        if (tid < c)
-            for (int qq = tid; qq < c; ++qq) acc += Ts[tid + qq * NBB] * (-tc * G[qq + c * NBB]);
-        __syncthreads();
-        if (tid < c) Ts[tid + c * NBB] = acc;
-        if (tid == 0) Ts[c + c * NBB] = tc;
-        __syncthreads();
+    if (warp < 2) {
+        const double* Gd = G + warp * (H * LD + H);
+        double* Td = Ts + warp * (H * LD + H);
+        double row[H];
+#pragma unroll
+        for (int c = 0; c < H; ++c) {
+            const int k = H * warp + c;
+            const double tc = k < b ? L.TAU[jb + k] : 0.0;
+            double s[2] = {0.0, 0.0};
+#pragma unroll
+            for (int p = 0; p < c; ++p) s[p & 1] = fma(row[p], Gd[p * LD + c], s[p & 1]);
+            row[c] = lane == c ? tc : (lane < c ? -tc * (s[0] + s[1]) : 0.0);
+            Td[c * LD + lane] = row[c];
+        }
     }
-    for (int e = tid; e < NBB * NBB; e += 256) Tq[e] = Ts[e];
+    __syncthreads();
+    // X = G12 T2, T12 = -T1 X: each warp two of the 4 x 4 tiles
+    double* X = Vs;                    // X(p, c) at X[c * LDX + p]
+    const int ti = warp >> 1;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int tj = 2 * (warp & 1) + u;
+        double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+        for (int k0 = 0; k0 < H; k0 += 4)
+            nrg::cta_dmma(d0, d1, G[(8 * ti + g) * LD + H + k0 + q4], Ts[(H + 8 * tj + g) * LD + H + k0 + q4]);
+        X[(8 * tj + 2 * q4) * LDX + 8 * ti + g] = d0;
+        X[(8 * tj + 2 * q4 + 1) * LDX + 8 * ti + g] = d1;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int tj = 2 * (warp & 1) + u;
+        double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+        for (int k0 = 0; k0 < H; k0 += 4)
+            nrg::cta_dmma(d0, d1, Ts[(k0 + q4) * LD + 8 * ti + g], X[(8 * tj + g) * LDX + k0 + q4]);
+        Ts[(H + 8 * tj + 2 * q4) * LD + 8 * ti + g] = -d0;
+        Ts[(H + 8 * tj + 2 * q4 + 1) * LD + 8 * ti + g] = -d1;
+    }
+    __syncthreads();
+    for (int e = tid; e < NBB * NBB; e += 256) Tq[e] = Ts[(e / NBB) * LD + e % NBB];
 }
 
 // Z(:, c0 .. c0+CBK-1) <- H_0 ... H_{n-2} Z(:, ...) panel by panel (last panel first), the
@@ -1037,12 +1083,11 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         auto apply_smem = [&](int c) {   // Z block (ld up to maxn + 15), two staging buffers, W and W2
             return sizeof(double) * ((size_t)(maxn + 15) * c + 2 * NBB * (NBB + 4) + 2 * NBB * c);
         };
-        const size_t prep_smem = sizeof(double) * (NBB * 65 + 2 * NBB * NBB);
         const int cbk = apply_smem(16) <= (size_t)optin ? 16 : (apply_smem(8) <= (size_t)optin ? 8 : 0);
         if (cbk > 0) {
             const int npan = (maxn - 2) / NBB + 1;
-            NRG_TRY(raise_smem_limit((const void*)k_bt_prep, prep_smem));
-            k_bt_prep<<<dim3(npan, ns), 256, prep_smem, st>>>(dsec, d_V, wsd, wsi);
+            NRG_TRY(raise_smem_limit((const void*)k_bt_prep, kBtPrepSmem));
+            k_bt_prep<<<dim3(npan, ns), 256, kBtPrepSmem, st>>>(dsec, d_V, wsd, wsi);
             int nblk = 0;
             for (int x = 0; x < ns; ++x) nblk += (secs[x].n + cbk - 1) / cbk;
             const size_t sm = apply_smem(cbk);
