@@ -948,7 +948,9 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
             const int n = secs[x].n, c = std::max(0, n - res_max);   // columns before the trailing block
             double* vec = wsd + secs[x].w_off + 3LL * n * n + 2LL * NB * n + n;
             double* A = d_V + secs[x].a_off;
-            if (c > 0) streamed.push_back(TriItem{A, vec, vec + n, vec + 2 * n, n, n, c});
+            // the streamed matrix moves to the space of Z and U, which the divide and conquer fills later
+            double* P = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(wsd + secs[x].w_off) + 127) & ~uintptr_t(127));
+            if (c > 0) streamed.push_back(TriItem{A, vec, vec + n, vec + 2 * n, n, n, c, P});
             items.push_back(TriItem{A + c + (long long)c * n, vec + c, vec + n + c, vec + 2 * n + c, n - c, n, 0});
         }
         NRG_TRY(tri_stream(ctx, streamed, tri_wide_clusters() ? 16 : 8, ctx->scratch.b[slot_base == 24 ? 48 : 49]));

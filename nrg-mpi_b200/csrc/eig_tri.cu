@@ -558,17 +558,22 @@ __global__ void __launch_bounds__(kTriThreads, 1) k_tri_res(const TriTask* __res
 // (FP64 MMA, inner length 2 NBS).  The sums that arrive are those of the matrix as stored:
 //   a = A(k, :) - sum_q (u_q(k) w_q + w_q(k) u_q),   y = A x - sum_q (u_q (w_q.x) + w_q (u_q.x)),
 // with w_q.x and u_q.x from a run of rows per block, sent beside the column sums: still one
-// message per step.  Bound by the L2 stream of a block (8 m^2 / CL bytes per step, m the
-// trailing order, at 37 of the 44..48 bytes per cycle that eight warps reach) and, below m
-// of about 600, by the chain of the step.  Order 1225: 9.8 ms to order 512 and 1.1 ms on
-// chip, against 17.2 ms of the cluster kernel with panels of 32 columns and two cluster
+// message per step.  The first such pass moves the matrix to columns that start on 128 bytes
+// (odd orders put every other column off by 8, and a load of a warp then touches a line more:
+// 10.0 against 9.3 thousand cycles for a product of order 870 on average); the last one brings
+// the trailing block back.  Bound by the L2 stream of a block (8 m^2 / CL bytes per step, m the
+// trailing order, at 40 of the 44..48 bytes per cycle that eight warps reach) and, below m
+// of about 600, by the chain of the step.  Order 1225: 9.1 ms to order 512 (9.8 before the
+// aligned columns and the 16 x 8 x 8 MMA on row pairs) and 1.1 ms on chip, against 17.2 ms of the cluster kernel with panels of 32 columns and two cluster
 // barriers per column that it replaced (8 blocks; with 16 that one was no faster).
 constexpr int kStreamSlots = 7;   // kept updates at most (NBS), fewer where they do not fit
 
 struct StreamTask {
-    double *A, *D, *E, *TAU;
-    int n, stop, rank, keep;   // stop: columns to reduce; keep: updates kept back
+    double *A, *D, *E, *TAU, *P;   // P: n columns of stream_ld(n), 128-byte aligned
+    int n, stop, rank, keep;       // stop: columns to reduce; keep: updates kept back
 };
+
+__host__ __device__ inline int stream_ld(int n) { return (n + 1 + 15) & ~15; }
 
 struct StreamLayout {
     int ld, nr, cols, keep;
@@ -686,6 +691,8 @@ __device__ __forceinline__ void stream_steps(const StreamTask& t, double* sm, un
     auto first_own = [&](int i0) { return (i0 - rank + CL - 1) / CL; };
     auto ex = [&](int i) { return (int)((unsigned)i % CL) * lay.cols + (int)((unsigned)i / CL); };
     int np = 0;                            // kept updates (complete pairs), u_q and w_q in slot q
+    const int ldp = stream_ld(n);
+    bool packed = true;                    // the matrix is still in A
     bool late = false;
     for (int k = 0; k <= t.stop; ++k) {
         const int b = k & 1;
@@ -770,34 +777,40 @@ __device__ __forceinline__ void stream_steps(const StreamTask& t, double* sm, un
                 U[nw + i] = i == k + 1 ? 0.0 : x;
             }
         }
-        if (tid == 0) {
-            if (fin) {
-                // the last reflector's entries at row k, which stays in the trailing block
+        if (fin) {
+            // the last reflector's entries at row k, which stays in the trailing block
+            if (tid == 0) {
                 U[cur + k] = h;
                 W[cur + k] = wpiv;
-            } else {
-                U[nw + k] = 0.0;       // a product that starts one row early to pair the rows
             }
+        } else if (tid < 16 && tid <= k) {
+            U[nw + k - tid] = 0.0;     // a product that starts up to 15 rows early
         }
         step_sync();
         // ---- 2. products with the new column; every warp keeps its own columns, warp + 8 i of
         // the block's ----
         const double* xs = U + nw;
         const int r0 = fin ? k : k + 1, mR = first_own(r0);
+        const int lds = packed ? n : ldp, rs = r0 - ((r0 + par) & (packed && !(apply && full > 0) ? 1 : 15));
+        const double* src = packed ? t.A : t.P + par;
         const int mw = mR + ((warp - mR) & (kTriWarps - 1));           // the warp's first live column
         if (apply && full > 0) {
-            // the kept updates go into the matrix on the way: 8 columns x 64 rows at a time as
-            // MMA accumulators, the next rows' entries loaded meanwhile; rows and columns
-            // beyond the end repeat the last one and are not stored
+            // the kept updates go into the matrix on the way: 8 columns x RU rows at a time as MMA
+            // accumulators, the next rows' entries loaded meanwhile.  Row 2 g + h of 16 rows is
+            // row g of tile h, so that a lane loads and stores row pairs.  Rows before the trailing
+            // block's are dead storage, rows and columns beyond the end are not stored.
+            constexpr int TU = 4, RU = 16 * TU;
             const int g = lane >> 2, q4 = lane & 3;
+            double* dst = fin ? t.A : t.P + par;
+            const int ldd = fin ? n : ldp;
             int pa[4], pb[4];              // offsets in shared memory
             bool have[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int q = 4 * e + q4, at = (q < full ? q : q - full) * ld + par;
                 have[e] = q < 2 * full;
-                pa[e] = have[e] ? (q < full ? lay.u() : lay.w()) + at : 0;
-                pb[e] = have[e] ? (q < full ? lay.w() : lay.u()) + at : 0;
+                pa[e] = (have[e] ? (q < full ? lay.u() : lay.w()) + at : par) + 2 * g;
+                pb[e] = have[e] ? (q < full ? lay.w() : lay.u()) + at : par;
             }
             for (int m0 = mw; m0 < cnt; m0 += 8 * kTriWarps) {
                 const int lb = rank + CL * min(m0 + kTriWarps * g, cnt - 1);
@@ -805,56 +818,89 @@ __device__ __forceinline__ void stream_steps(const StreamTask& t, double* sm, un
 #pragma unroll
                 for (int e = 0; e < 4; ++e) bf[e] = have[e] ? -sm[pb[e] + lb] : 0.0;
                 const int mc0 = m0 + 2 * kTriWarps * q4, mc1 = mc0 + kTriWarps;
-                double* c0 = t.A + (size_t)(rank + CL * min(mc0, cnt - 1)) * n;
-                double* c1 = t.A + (size_t)(rank + CL * min(mc1, cnt - 1)) * n;
+                const size_t j0 = rank + CL * min(mc0, cnt - 1), j1 = rank + CL * min(mc1, cnt - 1);
+                const double *c0 = src + j0 * lds + 2 * g, *c1 = src + j1 * lds + 2 * g;
+                double *d0 = dst + j0 * ldd + 2 * g, *d1 = dst + j1 * ldd + 2 * g;
                 double s0 = 0.0, s1 = 0.0;
-                auto fetch = [&](int R, double (&x)[8][2]) {
-                    if (R + 64 <= n) {
+                auto fetch = [&](int R, double2 (&x)[TU][2]) {
+                    const double *p0 = c0 + R, *p1 = c1 + R;
+                    if (R + RU <= n) {
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) {
-                            x[u][0] = c0[R + g + 8 * u];
-                            x[u][1] = c1[R + g + 8 * u];
+                        for (int u = 0; u < TU; ++u) {
+                            x[u][0] = *reinterpret_cast<const double2*>(p0 + 16 * u);
+                            x[u][1] = *reinterpret_cast<const double2*>(p1 + 16 * u);
                         }
                     } else {
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) {
-                            x[u][0] = c0[min(R + g + 8 * u, n - 1)];
-                            x[u][1] = c1[min(R + g + 8 * u, n - 1)];
+                        for (int u = 0; u < TU; ++u) {
+                            const int i = R + 2 * g + 16 * u;
+                            x[u][0] = x[u][1] = make_double2(0.0, 0.0);
+                            if (i + 1 < n) {
+                                x[u][0] = *reinterpret_cast<const double2*>(p0 + 16 * u);
+                                x[u][1] = *reinterpret_cast<const double2*>(p1 + 16 * u);
+                            } else if (i < n) {
+                                x[u][0].x = p0[16 * u];
+                                x[u][1].x = p1[16 * u];
+                            }
                         }
                     }
                 };
-                auto apply_at = [&](int R, double (&x)[8][2]) {
-                    const int last = n - 1;
+                const bool in0 = mc0 < cnt, in1 = mc1 < cnt;
+                auto apply_at = [&](int R, double2 (&x)[TU][2]) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
+                    for (int e = 0; e < 4; e += 2)
                         if (4 * e < 2 * full) {
+                            // beyond n it reads on into what follows the vector: rows that are not kept
+                            const double *lo = sm + pa[e] + R, *hi = sm + pa[e + 1] + R;
 #pragma unroll
-                            for (int u = 0; u < 8; ++u)
-                                nrg::cta_dmma(x[u][0], x[u][1], sm[pa[e] + min(R + g + 8 * u, last)], bf[e]);
+                            for (int u = 0; u < TU; ++u)
+                                nrg::cta_dmma16(x[u][0].x, x[u][1].x, x[u][0].y, x[u][1].y,
+                                                *reinterpret_cast<const double2*>(lo + 16 * u),
+                                                *reinterpret_cast<const double2*>(hi + 16 * u), bf[e], bf[e + 1]);
                         }
+                    double *o0 = d0 + R, *o1 = d1 + R;
+                    const double* xr = xs + R + 2 * g;
+                    if (R + RU <= n && !(fin && R == rs)) {
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int i = R + g + 8 * u;
-                        if (i < n) {
-                            if (mc0 < cnt) c0[i] = x[u][0];
-                            if (mc1 < cnt) c1[i] = x[u][1];
-                            const double xv = fin ? 0.0 : xs[i];
-                            s0 = fma(x[u][0], xv, s0);
-                            s1 = fma(x[u][1], xv, s1);
+                        for (int u = 0; u < TU; ++u) {
+                            if (in0) *reinterpret_cast<double2*>(o0 + 16 * u) = x[u][0];
+                            if (in1) *reinterpret_cast<double2*>(o1 + 16 * u) = x[u][1];
+                            const double2 xv = *reinterpret_cast<const double2*>(xr + 16 * u);
+                            s0 = fma(x[u][0].y, xv.y, fma(x[u][0].x, xv.x, s0));
+                            s1 = fma(x[u][1].y, xv.y, fma(x[u][1].x, xv.x, s1));
+                        }
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < TU; ++u) {
+                            const int i = R + 2 * g + 16 * u;
+                            if (i + 1 < n) {
+                                const bool kept = !fin || i + 1 >= r0;
+                                if (kept && in0) *reinterpret_cast<double2*>(o0 + 16 * u) = x[u][0];
+                                if (kept && in1) *reinterpret_cast<double2*>(o1 + 16 * u) = x[u][1];
+                                const double2 xv = *reinterpret_cast<const double2*>(xr + 16 * u);
+                                s0 = fma(x[u][0].y, xv.y, fma(x[u][0].x, xv.x, s0));
+                                s1 = fma(x[u][1].y, xv.y, fma(x[u][1].x, xv.x, s1));
+                            } else if (i < n) {
+                                if (in0) o0[16 * u] = x[u][0].x;
+                                if (in1) o1[16 * u] = x[u][1].x;
+                                s0 = fma(x[u][0].x, xr[16 * u], s0);
+                                s1 = fma(x[u][1].x, xr[16 * u], s1);
+                            }
                         }
                     }
-                    if (R == r0 && g == 0 && !fin) {   // row k + 1
-                        if (mc0 < cnt) rowv[mc0] = x[0][0];
-                        if (mc1 < cnt) rowv[mc1] = x[0][1];
+                    if (R == rs && g == (r0 - rs) >> 1 && !fin) {   // row k + 1
+                        const bool odd = (r0 - rs) & 1;
+                        if (in0) rowv[mc0] = odd ? x[0][0].y : x[0][0].x;
+                        if (in1) rowv[mc1] = odd ? x[0][1].y : x[0][1].x;
                     }
                 };
-                double x[8][2], y[8][2];
-                fetch(r0, x);
-                for (int R = r0; R < n; R += 128) {
-                    if (R + 64 < n) fetch(R + 64, y);
+                double2 x[TU][2], y[TU][2];
+                fetch(rs, x);
+                for (int R = rs; R < n; R += 2 * RU) {
+                    if (R + RU < n) fetch(R + RU, y);
                     apply_at(R, x);
-                    if (R + 128 < n) fetch(R + 128, x);
-                    if (R + 64 < n) apply_at(R + 64, y);
+                    if (R + 2 * RU < n) fetch(R + 2 * RU, x);
+                    if (R + RU < n) apply_at(R + RU, y);
                 }
 #pragma unroll
                 for (int o = 4; o < 32; o <<= 1) {
@@ -862,21 +908,21 @@ __device__ __forceinline__ void stream_steps(const StreamTask& t, double* sm, un
                     s1 += __shfl_xor_sync(kAll, s1, o);
                 }
                 if (g == 0 && !fin) {
-                    if (mc0 < cnt) part[mc0] = s0;
-                    if (mc1 < cnt) part[mc1] = s1;
+                    if (in0) part[mc0] = s0;
+                    if (in1) part[mc1] = s1;
                 }
             }
+            packed = false;
         } else {
             // three columns at a time in parts of 256 rows, 16-byte loads of row pairs, the next
             // part's loads in flight.  Pairs beyond the end repeat the last whole one against a
             // zero; the last row is taken by itself when it has no partner.
-            const int rs = (k + 1) - ((k + 1 + par) & 1);
             const int pend = rs + 2 * ((n - rs) / 2);                  // end of the whole pairs
             for (int m0 = mw; m0 < cnt; m0 += 3 * kTriWarps) {
                 const double* col[3];
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
-                    col[c] = t.A + (size_t)(rank + CL * min(m0 + kTriWarps * c, cnt - 1)) * n + 2 * lane;
+                    col[c] = src + (size_t)(rank + CL * min(m0 + kTriWarps * c, cnt - 1)) * lds + 2 * lane;
                 auto fetch = [&](int R, double2 (&x)[3][4]) {
                     if (R + 256 <= pend) {
 #pragma unroll
@@ -905,13 +951,14 @@ __device__ __forceinline__ void stream_steps(const StreamTask& t, double* sm, un
                 };
                 double2 x[3][4], y[3][4];
                 fetch(rs, x);
-                if (lane == 0) {               // row k + 1 of these columns
+                if (lane == (r0 - rs) >> 1) {  // row k + 1 of these columns
 #pragma unroll
                     for (int c = 0; c < 3; ++c)
-                        if (m0 + kTriWarps * c < cnt) rowv[m0 + kTriWarps * c] = rs == k + 1 ? x[c][0].x : x[c][0].y;
-                    if (pend < n)
+                        if (m0 + kTriWarps * c < cnt) rowv[m0 + kTriWarps * c] = (r0 - rs) & 1 ? x[c][0].y : x[c][0].x;
+                }
+                if (lane == 0 && pend < n) {
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) sum[c] = col[c][n - 1] * xs[n - 1];
+                    for (int c = 0; c < 3; ++c) sum[c] = col[c][n - 1] * xs[n - 1];
                 }
                 for (int R = rs; R < pend; R += 512) {
                     if (R + 256 < pend) fetch(R + 256, y);
@@ -1111,7 +1158,7 @@ int tri_stream(nrg_context* ctx, const std::vector<TriItem>& items, int CL, DevB
         int keep = kStreamSlots;
         while (keep > 1 && 8LL * StreamLayout(it.n, CL, keep).doubles(CL) > kSmemMax) --keep;
         smem = std::max(smem, sizeof(double) * (size_t)StreamLayout(it.n, CL, keep).doubles(CL));
-        for (int r = 0; r < CL; ++r) tasks.push_back(StreamTask{it.A, it.D, it.E, it.TAU, it.n, it.stop, r, keep});
+        for (int r = 0; r < CL; ++r) tasks.push_back(StreamTask{it.A, it.D, it.E, it.TAU, it.P, it.n, it.stop, r, keep});
     }
     if (smem > (size_t)kSmemMax) {
         nrg_set_error_message("order %d exceeds the streamed tridiagonalisation", items[0].n);

@@ -306,6 +306,7 @@ struct TriItem {
     double* A;             // full symmetric storage, leading dimension lda
     double *D, *E, *TAU;
     int n, lda, stop;
+    double* P = nullptr;   // tri_stream: workspace of n ((n + 16) & ~15) doubles, 128-byte aligned
 };
 int tri_resident_max();
 bool tri_wide_clusters();   // clusters of 16 blocks can be placed
