@@ -9,7 +9,7 @@
 //   kept energies: tables.cu); the host keeps the sector-level tables it sizes the
 //   launches with (a few integers per sector and operation cross per iteration).  Models
 //   whose operations change the quantum numbers alike (ties in sortBasisArray) build the
-//   records on the host, with the exchange sort replayed;
+//   records on the host, in the exchange sort's order;
 // * host drop-in (host_drop_in = 1): every routine goes through its public entry point
 //   with host arrays, exactly as the Fortran caller would call the drop-in: module arrays
 //   live in host memory and cross to the device and back at every call.
@@ -88,89 +88,63 @@ bool bucket_order(const std::vector<int>& rec, int n, int nVar, std::vector<int>
     return true;
 }
 
-// One pass i of the exchange sequence on ranks R (ids I carried along): the carried key
-// is swapped with every strictly smaller key after position i, until it is the pass's
-// target (the i-th smallest key), after which no key can be smaller.  ready(e) returns
-// once the positions below e hold the previous pass's result; publish(j) announces that
-// this pass is done with the positions below j.
-template <class Ready, class Publish>
-void exchange_pass(int* R, int* I, int n, int i, int t, Ready&& ready, Publish&& publish) {
-    ready(i + 1);
-    int c = R[i], ci = I[i];
-    int j = i + 1;
-    while (c > t && j < n) {
-        ready(std::min(n, j + 256));
-        const int stop = std::min(n, j + 256);
-        while (c > t && j < stop) {
-            // skip keys not smaller than the carried one, eight at a time
-            while (j + 8 <= stop) {
-                int m = 0;
-                for (int u = 0; u < 8; ++u) m |= R[j + u] < c;
-                if (m) break;
-                j += 8;
-            }
-            for (const int end = std::min(stop, j + 8); c > t && j < end; ++j) {
-                const int x = R[j];
-                if (x < c) {
-                    R[j] = c;
-                    c = x;
-                    const int xi = I[j];
-                    I[j] = ci;
-                    ci = xi;
-                }
-            }
-        }
-        publish(j);
+// Final order of the exchange sort (for every i, for every j > i: swap when the key at j is smaller)
+// on integer ranks, 0 .. nrank - 1: I[i] is the initial position of the record that ends at i.
+//
+// Position j keeps the larger of its own key and each key carried past it, and passes the smaller
+// one on; so what the passes before j carry past it is the sorted list of the records before
+// j, and j inserts its own.  In that list the inserted record goes behind those of equal rank,
+// and a run of a larger rank that comes by turns by one: its first record is held until a
+// larger key arrives, while the others of the run pass it.  The order within a rank thus follows
+// from the number of smaller records inserted between its own, taken backwards from the end:
+// undo the turns, take away the last record.  O(n log n); replaying the swaps of 9600 records
+// takes 224 ms in random order (59 in descending), this 0.6.
+void exchange_order(const std::vector<int>& rank, int nrank, std::vector<int>* I) {
+    const int n = (int)rank.size();
+    std::vector<int> start(nrank + 1, 0), fill(nrank), member(n), less(n), tree;
+    for (int r : rank) start[r + 1]++;
+    for (int r = 0; r < nrank; ++r) start[r + 1] += start[r];
+    std::copy(start.begin(), start.end() - 1, fill.begin());
+    // the records of every rank in their initial order, and for each the smaller ones before it
+    tree.assign(nrank + 1, 0);
+    for (int j = 0; j < n; ++j) {
+        int c = 0;
+        for (int x = rank[j]; x > 0; x -= x & -x) c += tree[x];
+        const int at = fill[rank[j]]++;
+        member[at] = j;
+        less[at] = c;
+        for (int x = rank[j] + 1; x <= nrank; x += x & -x) tree[x]++;
     }
-    R[i] = c;
-    I[i] = ci;
-}
-
-// All passes of the exchange sequence.  Large inputs run consecutive passes on several
-// host threads in a wavefront: pass i+1 reads a position only after pass i has moved past
-// it (an acquire/release progress word per thread, tagged with the pass number), so every
-// swap is the one the serial sequence makes, in the same order per position.
-void exchange_replay(int* R, int* I, const int* target, int n) {
-    const unsigned hw = std::thread::hardware_concurrency();
-    const int T = (int)std::min<unsigned>(8, hw ? hw : 1);
-    if (n < 16384 || T < 2) {
-        for (int i = 0; i < n; ++i)
-            exchange_pass(R, I, n, i, target[i], [](int) {}, [](int) {});
-        return;
-    }
-    // progress word of the pass a thread runs: (pass + 1) << 32 | first position not done
-    std::vector<std::atomic<uint64_t>> prog(T);
-    for (auto& p : prog) p.store(0, std::memory_order_relaxed);
-    auto worker = [&](int k) {
-        for (int i = k; i < n; i += T) {
-            std::atomic<uint64_t>& mine = prog[k];
-            std::atomic<uint64_t>& prev = prog[(k + T - 1) % T];
-            int known = i == 0 ? n : 0;      // positions the previous pass is done with
-            auto ready = [&](int e) {
-                for (int spins = 0; known < e; ++spins) {
-                    const uint64_t v = prev.load(std::memory_order_acquire);
-                    const long long pass = (long long)(v >> 32) - 1;
-                    known = pass > i - 1 ? n : (pass == i - 1 ? (int)(uint32_t)v : 0);
-                    if (known < e && spins > 64) std::this_thread::yield();
+    I->resize(n);
+    for (int r = 0; r < nrank; ++r) {
+        const int s0 = start[r], m = start[r + 1] - s0;
+        int top = 1;
+        while (2 * top <= m) top *= 2;
+        tree.assign(m + 1, 0);   // the free slots
+        for (int x = 1; x <= m; ++x) tree[x] = x & -x;
+        int head = 0, after = s0;   // first record's place among the free slots; smaller records in the end
+        for (int t = m - 1; t >= 0; --t) {
+            const int size = t + 1, turns = (after - less[s0 + t]) % size;
+            after = less[s0 + t];
+            head = (head + size - turns) % size;
+            int k = (head + size - 1) % size;   // the last record's place
+            if (k < head) --head;
+            if (head == size - 1) head = 0;
+            int slot = 0;
+            for (int b = top; b > 0; b >>= 1)
+                if (slot + b <= m && tree[slot + b] <= k) {
+                    slot += b;
+                    k -= tree[slot];
                 }
-            };
-            auto publish = [&](int j) {
-                mine.store(((uint64_t)(i + 1) << 32) | (uint32_t)j, std::memory_order_release);
-            };
-            publish(i + 1);
-            exchange_pass(R, I, n, i, target[i], ready, publish);
-            publish(n);
+            (*I)[s0 + slot] = member[s0 + t];
+            for (int x = slot + 1; x <= m; x += x & -x) tree[x]--;
         }
-    };
-    std::vector<std::thread> pool;
-    for (int k = 1; k < T; ++k) pool.emplace_back(worker, k);
-    worker(0);
-    for (auto& th : pool) th.join();
+    }
 }
 
 // sortBasisArray (module.F90:531-602): exchange sort of whole records.  When no two
 // records share (basis, reference) any correct sort gives its result; otherwise the
-// order among equal keys is the exchange sequence's, which is replayed.
+// order among equal keys is the exchange sort's (exchange_order).
 void sort_basis(std::vector<int>& rec, int n, int nVar) {
     const int rs = nVar + 3;
     auto greater = [&](const int* a, const int* b) {
@@ -199,20 +173,13 @@ void sort_basis(std::vector<int>& rec, int n, int nVar) {
         rec.swap(out);
         return;
     }
-    // The exchange sequence on integer ranks of the keys (equal keys, equal ranks) with
-    // the records' ids carried along.  Pass i carries the smallest key seen so far and
-    // swaps it with every strictly smaller key after it; it ends once the carried key is
-    // the i-th smallest of all (known from the stable sort above), since no key after it
-    // can then be smaller: the same swaps as the full scan, without the tail.
-    std::vector<int> rk(n), id(n), target(n);
-    for (int k = 0, r = -1; k < n; ++k) {
+    std::vector<int> rk(n), I;
+    int r = -1;
+    for (int k = 0; k < n; ++k) {
         if (k == 0 || greater(&rec[(size_t)idx[k] * rs], &rec[(size_t)idx[k - 1] * rs])) ++r;
         rk[idx[k]] = r;
-        target[k] = r;
     }
-    std::iota(id.begin(), id.end(), 0);
-    exchange_replay(rk.data(), id.data(), target.data(), n);
-    const int* I = id.data();
+    exchange_order(rk, r + 1, &I);
     std::vector<int> out((size_t)n * rs);
     for (int i = 0; i < n; ++i) std::memcpy(&out[(size_t)i * rs], &rec[(size_t)I[i] * rs], sizeof(int) * rs);
     rec.swap(out);

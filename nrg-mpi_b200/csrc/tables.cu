@@ -26,7 +26,7 @@
 // whole runs (old sector s, operation a) in increasing s: the sector table follows from
 // the (s, a) pairs alone, and the records and (sector, operation) row lists are written
 // per row by one kernel.  Models whose operations share quantum numbers (the two-orbital
-// model) keep the host replay of the exchange sort.
+// model) build the records on the host, in the exchange sort's order of equal keys.
 #include "internal.hpp"
 
 #include <algorithm>
