@@ -362,9 +362,15 @@ __global__ void __launch_bounds__(256) k_broaden(const double* __restrict__ bins
     const double* E = bins + (size_t)m * nbin;
     const double* W = bins + ld + (size_t)m * nbin;
     double s = 0.0;
+    // beyond |ln(w/E)| = 27.5 b the exponential is exactly zero (exp(-756)): such a bin is left out
+    // before its divisions, logarithm and exponential, unless its weight is not finite.  Bound by
+    // FP64 arithmetic; 801 frequencies at b = 0.6 take 0.24 ms in all, 0.29 with every bin evaluated.
+    const double wa = fabs(w), far = exp(27.5 * b), near = exp(-27.5 * b);
     for (int i = threadIdx.x; i < nbin; i += blockDim.x) {
         const double wi = W[i], ei = E[i];
         if (wi == 0.0 || !(w * ei > 0.0)) continue;
+        const double ea = fabs(ei);
+        if ((wa > ea * far || wa < ea * near) && fabs(wi) < INFINITY) continue;
         const double x = log(w / ei) / b;
         s += wi * exp(-x * x) / fabs(ei);
     }
