@@ -19,12 +19,12 @@ second (60 per step), whole job.
   copies its module arrays host->device and back, as a Fortran caller would), with the
   caller's arrays page-locked; e2e.pageable: the same with pageable arrays (a Fortran
   allocatable), which the routines copy whole.
-* roofline: the kernel with the largest share of device time, k_tri_cluster (Householder
-  tridiagonalisation of the sectors of order > 128): algorithmic flops sum_s 4/3 d_s^3
+* roofline: the kernels with the largest share of device time, k_tri_stream and k_tri_res
+  (Householder tridiagonalisation of the sectors of order > 128): algorithmic flops sum_s 4/3 d_s^3
   per launch over its event-timed launch duration, against a cuBLAS DGEMM peak measured
-  here (the FP64 ceiling; tcgen05 has no FP64 kind); traffic = DRAM bytes per launch of an
-  ncu capture of this workload, read from profiles/roofline_traffic.json (null without
-  it).  "eigensolver" gives the same for the whole eigensolver of an iteration
+  here (the FP64 ceiling; tcgen05 has no FP64 kind); traffic = DRAM bytes per launch pair of
+  an ncu capture of the largest class's order, read from profiles/roofline_traffic.json (null
+  without it).  "eigensolver" gives the same for the whole eigensolver of an iteration
   (sum_s (4/3+2) d_s^3 over the event-timed window).
 * cpu_baseline: the oracle (numpy/scipy port of the reference path, OpenBLAS on all host
   threads) on two full-size iterations of the same chain with their backward density
@@ -390,7 +390,7 @@ def oracle_window(n_full, warmup=0):
 
 
 def roofline_traffic():
-    """DRAM bytes per launch of the roofline kernel on this workload (ncu), if captured."""
+    """DRAM bytes per launch pair of the roofline kernels (ncu), if captured."""
     try:
         with open(TRAFFIC_FILE) as f:
             t = json.load(f)
@@ -625,7 +625,7 @@ def main():
             "device_memory_gb": device_gb,
             "sum_rule": sums,
             "gpu_launches": int(launches),
-            "roofline": {"kernel": "k_tri_cluster (FP64 Householder tridiagonalisation of the sectors of "
+            "roofline": {"kernel": "k_tri_stream + k_tri_res (FP64 Householder tridiagonalisation of the sectors of "
                                    "order > 128, one thread-block cluster per sector)",
                          "bound": "tensor", "pipe": "fp64",
                          "achieved": tri_ach, "peak": peak, "unit": "TFLOP/s",
