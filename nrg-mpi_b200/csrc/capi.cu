@@ -529,6 +529,16 @@ int nrg_context_set_model(nrg_context* ctx, const nrg_model* m) {
     return NRG_OK;
 }
 
+// The solver of nrg_diagonalization; NRG_ENTRY_SOLVER=device (read once per process) takes the
+// device-resident runs', for a caller that compares no signs and for tests.
+static EigSolver entry_solver() {
+    static const EigSolver solver = [] {
+        const char* e = getenv("NRG_ENTRY_SOLVER");
+        return e && !std::strcmp(e, "device") ? EigSolver::Device : EigSolver::Panel;
+    }();
+    return solver;
+}
+
 // ------------------------------------------------------------------------------------
 int nrg_diagonalization(nrg_context* ctx, int32_t iteration, const nrg_diagonalization_io* io) {
     NRG_TRY(need_model(ctx));
@@ -596,6 +606,7 @@ int nrg_diagonalization(nrg_context* ctx, int32_t iteration, const nrg_diagonali
     DiagOut out;
     // a page-locked eigenvector array takes each group's blocks as soon as they are final
     DiagPost post;
+    post.solver = entry_solver();
     if (rc == NRG_OK && dV != io->eigenvector) {
         cudaPointerAttributes a;
         if (cudaPointerGetAttributes(&a, io->eigenvector) == cudaSuccess && a.type == cudaMemoryTypeHost)

@@ -62,4 +62,6 @@ __host__ __device__ inline long long syev_vec_off(long long n) {
 
 // launch helpers implemented in the .cu files (return NRG status)
 int launch_tri_small(const SyevSector* d_secs, int nsec, double* eigbuf, double* wsd, int* d_status, cudaStream_t st);
+// orders <= 128, one block each: eig_panel.cu's solver
+int launch_syev_panel(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* d_status, cudaStream_t st);
 int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* wsi, int* d_status, cudaStream_t st);

@@ -13,66 +13,21 @@
 //      final order) with the eigenvector update Z(:, kept) * U as a grouped GEMM;
 //   3. back-transformation in panels of 64 reflectors: Gram matrix and V^T Z as grouped
 //      GEMMs, the triangular factor T in one block, then Z -= (V T)(V^T Z).
+//
+// That is the solver of the runs that keep their eigenvectors on the device.  For eigenvectors
+// that go to a caller (EigSolver::Panel) steps 1 and 2 are those of eig_panel.cu.
 #include "eig_dc.cuh"
+#include "eig_sector.cuh"
 #include "internal.hpp"
-
 
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
 
-
 namespace {
 
-constexpr int NB = 32;        // tridiagonalisation panel
-constexpr int NBB = 64;       // back-transformation panel
-constexpr int DC_LOW = kDcLeafRows;   // merges of up to this many rows run inside one block
-constexpr int TPB = 256;
-constexpr int CB = 32;        // columns per block in the symmetric matrix-vector product
-
-struct LSec {
-    long long a_off, e_off, w_off, i_off;
-    int n;
-    int z_sel;   // where the divide and conquer leaves the eigenvectors: 0 Z, 2 Qt (in n x n)
-};
-
-// workspace per sector: Z, U, Qt (n x n each), the panel V | W (n x 2 NB), y, the D&C
-// vectors (16 n + 64), then the back-transformation's T factors and explicit reflector
-// panels ((n + NBB)^2 bounds both)
-long long lws_doubles(long long n) {
-    return 3 * n * n + 2LL * NB * n + n + 16 * n + 64 + (n + NBB) * (n + NBB);
-}
-long long lws_ints(long long n) { return 12 * n + 64; }
-
-struct LView {
-    double *A, *Z, *U, *Qt, *ZV, *VW, *y, *vec, *D, *E, *TAU, *R;   // ZV: the eigenvectors of T
-    int* I;
-    Scratch S;
-    int n;
-};
-
-__device__ LView lview(const LSec& s, double* eigbuf, double* wsd, int* wsi) {
-    LView v;
-    const long long n = s.n, sq = n * n;
-    v.n = s.n;
-    v.A = eigbuf + s.a_off;
-    double* W = wsd + s.w_off;
-    v.Z = W;
-    v.U = W + sq;
-    v.Qt = W + 2 * sq;
-    v.ZV = W + s.z_sel * sq;
-    v.VW = W + 3 * sq;
-    v.y = v.VW + 2LL * NB * n;
-    v.vec = v.y + n;
-    v.D = v.vec;
-    v.E = v.vec + n;
-    v.TAU = v.vec + 2 * n;
-    v.R = v.vec + 16 * n + 64;
-    v.I = wsi + s.i_off;
-    v.S = scratch_at(v.vec, v.I, s.n);
-    return v;
-}
+static_assert(DC_LOW == kDcLeafRows, "the leaves of the divide and conquer");
 
 // ---------------------------------------------------------------------------------
 // tridiagonalisation
@@ -878,8 +833,9 @@ static bool tri_multi_kernel() {
     return multi;
 }
 
-int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V, double* d_E, int slot_base,
-               cudaEvent_t evals_ready) {
+int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V, double* d_E, EigSolver solver,
+               int slot_base, cudaEvent_t evals_ready) {
+    const bool panel = solver == EigSolver::Panel;
     const int ns = (int)in.size();
     if (ns == 0) return NRG_OK;
     cudaStream_t st = ctx->stream;
@@ -892,7 +848,7 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         secs[s].n = in[s].n;
         int levels = 0;
         for (int w = DC_LOW; w < in[s].n; w *= 2) ++levels;
-        secs[s].z_sel = levels % 2 ? 2 : 0;
+        secs[s].z_sel = !panel && levels % 2 ? 2 : 0;
         secs[s].w_off = wd;
         secs[s].i_off = wi;
         wd += lws_doubles(in[s].n);
@@ -913,7 +869,7 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
     // path is left: nbig sectors, the first ones (the list is sorted by decreasing order).
     const int res_max = tri_resident_max(), stream_max = tri_multi_kernel() ? 0 : tri_stream_max();
     int nbig = 0;
-    while (nbig < ns && secs[nbig].n > stream_max) ++nbig;
+    while (!panel && nbig < ns && secs[nbig].n > stream_max) ++nbig;
     NRG_TRY(h2d_async(ctx, bsec.p, secs.data(), sizeof(LSec) * ns));
     const LSec* dsec = bsec.as<LSec>();
     double* wsd = bwd.as<double>();
@@ -935,14 +891,17 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         NRG_TRY(raise_smem_limit((const void*)k_tri_symv, symv_smem));
 
     // ---- 1. tridiagonalisation ----
-    const bool clustered = nbig == 0;
     cudaEvent_t te[2] = {nullptr, nullptr};
     if (ctx->profiling) {
         NRG_CUDA_TRY(cudaEventCreate(&te[0]));
         NRG_CUDA_TRY(cudaEventCreate(&te[1]));
         NRG_CUDA_TRY(cudaEventRecord(te[0], st));
     }
-    {
+    if (panel) {
+        bool done = false;   // otherwise every sector takes the multi-kernel path
+        NRG_TRY(panel_tridiagonal(ctx, dsec, ns, maxn, d_V, wsd, wsi, &done));
+        nbig = done ? 0 : ns;
+    } else {
         std::vector<TriItem> items, streamed;
         for (int x = nbig; x < ns; ++x) {
             const int n = secs[x].n, c = std::max(0, n - res_max);   // columns before the trailing block
@@ -956,6 +915,7 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         NRG_TRY(tri_stream(ctx, streamed, tri_wide_clusters() ? 16 : 8, ctx->scratch.b[slot_base == 24 ? 48 : 49]));
         NRG_TRY(tri_resident(ctx, items, ctx->scratch.b[slot_base == 24 ? 46 : 47]));
     }
+    const bool clustered = nbig == 0;
     if (ctx->profiling) {
         NRG_CUDA_TRY(cudaEventRecord(te[1], st));
         if (clustered) {
@@ -1010,7 +970,9 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
     }
 
     // ---- 2. divide and conquer ----
-    {
+    if (panel) {
+        NRG_TRY(panel_merges(ctx, secs, dsec, maxn, d_V, wsd, wsi, bmrg, gslot));
+    } else {
         NRG_TRY(raise_smem_limit((const void*)k_dc_low, kLeafSmem));
         int nchunk = 0;
         for (int x = 0; x < ns; ++x) nchunk += (secs[x].n + DC_LOW - 1) / DC_LOW;
@@ -1021,7 +983,7 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
     // the eigenvectors alternate between Z and Qt from level to level (in units of n x n)
     long long z_in = 0, z_out = 2;
     NRG_TRY(raise_smem_limit((const void*)k_dc_prep, kPrepSmem));
-    for (int s = DC_LOW; s < maxn; s *= 2) {
+    for (int s = DC_LOW; !panel && s < maxn; s *= 2) {
         std::vector<Merge> ms;
         std::vector<GemmProblem> probs;
         int blk = 0, widest = 0;

@@ -288,13 +288,22 @@ int launch_ggemm(nrg_context* ctx, std::vector<GemmProblem>& probs, int scratch_
 
 
 
+// Which solver: Device, the faster one, for eigenvectors that stay on the device; Panel
+// (eig_panel.cu) for those that a caller receives, whose signs must not change from one
+// version of the code to the next.
+enum class EigSolver { Device, Panel };
+
 // eigensolver for sectors of order > 128 across the whole GPU (eig_large.cu); the
 // descriptors use a_off / e_off / n only
 // (scratch slots slot_base .. slot_base + 6; on ctx->stream)
 // evals_ready (optional) is recorded on ctx->stream once the eigenvalues are in d_E,
 // before the back-transformation
-int syev_large(nrg_context* ctx, const std::vector<SyevSector>& secs, double* d_V, double* d_E, int slot_base,
-               cudaEvent_t evals_ready = nullptr);
+int syev_large(nrg_context* ctx, const std::vector<SyevSector>& secs, double* d_V, double* d_E, EigSolver solver,
+               int slot_base, cudaEvent_t evals_ready = nullptr);
+struct LSec;
+int panel_tridiagonal(nrg_context* ctx, const LSec* dsec, int ns, int maxn, double* d_V, double* wsd, int* wsi, bool* done);
+int panel_merges(nrg_context* ctx, const std::vector<LSec>& secs, const LSec* dsec, int maxn, double* d_V, double* wsd,
+                 int* wsi, DevBuf& bmrg, int gslot);
 constexpr int kLargeSector = 128;
 
 // tridiagonalisation (eig_tri.cu) on ctx->stream: D, E, tau and the reflectors (below the
@@ -392,6 +401,7 @@ struct DiagPost {
     // returns with every block in h_V (the caller then copies nothing).
     double* h_V = nullptr;
     bool copied_V = false;                 // out: h_V holds the eigenvectors
+    EigSolver solver = EigSolver::Device;
 };
 int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eold, int nb_old,
                 const double* d_IMold, double* d_V, double* d_E, DiagOut* out, DiagPost* post = nullptr);

@@ -308,6 +308,7 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
     const bool early = post && post->early;
     double* h_E = post ? post->h_E : nullptr;
     TruncTables* trunc = post ? post->trunc : nullptr;
+    const EigSolver solver = post ? post->solver : EigSolver::Device;
     const int nsec = S.nsub;
     std::vector<int> order(nsec);
     std::iota(order.begin(), order.end(), 0);
@@ -395,17 +396,24 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
         NRG_CUDA_TRY(cudaStreamWaitEvent(s1, ctx->ev_fork, 0));
         cudaStream_t caller = ctx->stream;
         ctx->stream = s1;
-        rl = syev_large(ctx, g1, d_V, d_E, 24, early && !g1.empty() ? ctx->ev_evals_hi : nullptr);
+        rl = syev_large(ctx, g1, d_V, d_E, solver, 24, early && !g1.empty() ? ctx->ev_evals_hi : nullptr);
         ctx->stream = caller;
         NRG_CUDA_TRY(cudaEventRecord(ctx->ev_join_hi, s1));
     } else {
-        rl = syev_large(ctx, g1, d_V, d_E, 24);
+        rl = syev_large(ctx, g1, d_V, d_E, solver, 24);
     }
     if (fork_small) NRG_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
     if (nsec > nlarge && rl == NRG_OK) {
-        rl = launch_syev(bsec.as<SyevSector>() + nlarge, nsec - nlarge, d_V, d_E, bwd.as<double>(),
-                         bwi.as<int>(), ctx->d_status.as<int>(), fork_small ? ctx->aux : ctx->stream);
-        ctx->launches += 2;
+        const SyevSector* small = bsec.as<SyevSector>() + nlarge;
+        const cudaStream_t st = fork_small ? ctx->aux : ctx->stream;
+        int* d_status = ctx->d_status.as<int>();
+        if (solver == EigSolver::Panel) {
+            rl = launch_syev_panel(small, nsec - nlarge, d_V, d_E, bwd.as<double>(), d_status, st);
+            ctx->launches++;
+        } else {
+            rl = launch_syev(small, nsec - nlarge, d_V, d_E, bwd.as<double>(), bwi.as<int>(), d_status, st);
+            ctx->launches += 2;
+        }
     }
     if (fork_small) NRG_CUDA_TRY(cudaEventRecord(ctx->ev_join, ctx->aux));
     const bool has_g2 = fork_large && !g2.empty();
@@ -413,7 +421,7 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
         NRG_CUDA_TRY(cudaStreamWaitEvent(ctx->aux2, ctx->ev_fork, 0));
         cudaStream_t caller = ctx->stream;
         ctx->stream = ctx->aux2;
-        if (rl == NRG_OK) rl = syev_large(ctx, g2, d_V, d_E, 31, early ? ctx->ev_evals2 : nullptr);
+        if (rl == NRG_OK) rl = syev_large(ctx, g2, d_V, d_E, solver, 31, early ? ctx->ev_evals2 : nullptr);
         ctx->stream = caller;
         NRG_CUDA_TRY(cudaEventRecord(ctx->ev_join2, ctx->aux2));
     }
