@@ -62,6 +62,10 @@ __host__ __device__ inline long long syev_vec_off(long long n) {
 
 // launch helpers implemented in the .cu files (return NRG status)
 int launch_tri_small(const SyevSector* d_secs, int nsec, double* eigbuf, double* wsd, int* d_status, cudaStream_t st);
-// orders <= 128, one block each: eig_panel.cu's solver
-int launch_syev_panel(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* d_status, cudaStream_t st);
-int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* wsi, int* d_status, cudaStream_t st);
+// orders <= 128, one block each.  unsure (one sector; may be null): set to 1 where the signs or
+// the mixing of eigenvectors hang on the last bits, otherwise to 0.  launch_syev_panel
+// (eig_panel.cu) given it solves the sector only where it is set, from the block at `from`
+// (n x n, not overwritten here; null: in eigbuf as usual).
+int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* unsure, int* d_status, cudaStream_t st);
+int launch_syev_panel(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, const int* unsure,
+                      const double* from, int* d_status, cudaStream_t st);

@@ -25,8 +25,9 @@ static_assert(kThreads == kBtThreads, "the back-transformation's block");
 __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict__ secs,
                                                     double* __restrict__ eigbuf,
                                                     double* __restrict__ evals,
-                                                    double* __restrict__ wsd, int* status) {
+                                                    double* __restrict__ wsd, int* unsure, int* status) {
     extern __shared__ __align__(16) double sm[];
+    __shared__ int maybe;
     const SyevSector sec = secs[blockIdx.x];
     const int n = sec.n;
     const int tid = threadIdx.x, T = blockDim.x;
@@ -41,11 +42,12 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
         if (__syncthreads_or(bad)) {
             if (tid == 0) atomicOr(status, NRG_DEV_NONFINITE);
             for (int i = tid; i < n; i += T) ev[i] = __longlong_as_double(0x7ff8000000000000LL);
+            if (unsure && tid == 0) *unsure = 0;
             return;
         }
     }
     if (n == 1) {
-        if (tid == 0) { ev[0] = A[0]; A[0] = 1.0; }
+        if (tid == 0) { ev[0] = A[0]; A[0] = 1.0; if (unsure) *unsure = 0; }
         return;
     }
     double* W = wsd + sec.w_off;
@@ -56,21 +58,28 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
     double* TAU = vec + 2 * n;
 
     // ---- 2. divide and conquer on (Dd, Ee) -> eigenvalues in Dd, vectors in Z ----
-    dc_leaf(0, n, n, Dd, Ee, Z, sm, status);
+    if (tid == 0) maybe = 0;
+    dc_leaf(0, n, n, Dd, Ee, Z, sm, status, unsure ? &maybe : nullptr);   // (a barrier before its first merge)
     __syncthreads();
+    if (unsure) {
+        const double gap = kUnsureGap * fmax(fabs(Dd[0]), fabs(Dd[n - 1]));
+        for (int i = tid; i < n - 1; i += T)
+            if (Dd[i + 1] - Dd[i] <= gap) maybe = 1;
+    }
 
     // ---- 3. back-transformation, straight to the output ----
     back_transform(A, n, TAU, Z, sm);
     for (int i = tid; i < n; i += T) ev[i] = Dd[i];
+    if (unsure && tid == 0) *unsure = maybe;   // (back_transform has barriers before this)
 }
 
 }  // namespace
 
-int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* wsi, int* d_status, cudaStream_t st) {
+int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* unsure, int* d_status, cudaStream_t st) {
     if (nsec == 0) return NRG_OK;
     NRG_TRY(launch_tri_small(d_secs, nsec, eigbuf, wsd, d_status, st));
     NRG_TRY(nrg::raise_smem_limit((const void*)k_syev, kLeafSmem));
-    k_syev<<<nsec, kThreads, kLeafSmem, st>>>(d_secs, eigbuf, evals, wsd, d_status);
+    k_syev<<<nsec, kThreads, kLeafSmem, st>>>(d_secs, eigbuf, evals, wsd, unsure, d_status);
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
 }

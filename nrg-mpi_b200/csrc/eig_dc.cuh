@@ -294,9 +294,16 @@ __device__ __forceinline__ MergeSize merge_size(const int* cnt, int nn, int n1) 
 // One merge of the children [a, a + s) and [a + s, b) up to the rank-one eigenvectors U (row
 // k, column a + j; rows ordered by child, not normalised: 1 / norm in rn) and the places of
 // the results.  b == a: no merge, but the barriers are taken.
+//
+// unsure (may be null): set when the merge decides close to its tolerance, or between values so
+// close (relative to the largest) that their eigenvectors hang on the last bits.  Of blocks of
+// order 128 with random entries 1 in 3,000 decides otherwise than the panel solver; the z of the
+// two differ by 0.3% of the tolerance there, so a quarter is a wide margin: it marks 10% of
+// them, a factor of 8 would mark 60%.
+constexpr double kUnsure = 1.25, kUnsureGap = 1e-6;
 template <class G>
 __device__ void leaf_merge(const G& g, int a, int s, int b, const Leaf& L, const double* Zc, double* U, double* red,
-                           unsigned* words, int* status) {
+                           unsigned* words, int* status, int* unsure) {
     const int t = g.rank(), T = g.size();
     const int nn = b - a, n1 = s;                       // nn > s, or 0
     const double beta = L.E[a + s - 1];
@@ -334,6 +341,12 @@ __device__ void leaf_merge(const G& g, int a, int s, int b, const Leaf& L, const
     g.sync();
     // ---- deflation: negligible z, then close neighbours among the others ----
     const bool in = t < nn;
+    if (unsure && in) {
+        const double zr = rho * fabs(zs[t]);
+        if ((zr > tol / kUnsure && zr < tol * kUnsure) ||
+            (t > 0 && ds[t] - ds[t - 1] <= kUnsureGap / (8.0 * kEps) * tol))
+            *unsure = 1;
+    }
     unsigned live[4], close[4];
     g.flags(in && rho * fabs(zs[in ? t : 0]) > tol, live, words);
     const bool kept = in && ((live[(t >> 5) & 3] >> (t & 31)) & 1u);
@@ -487,7 +500,7 @@ __device__ __forceinline__ void leaf_deflated(int t, int T, int a, int s, int nn
 
 // the levels of one warp's 32 rows: merges of W = 2 s rows, 32 / W at a time
 template <int W>
-__device__ void warp_level(int r0, int nl, const Leaf& L, double* area, double* Zg, long long ldz, int* status) {
+__device__ void warp_level(int r0, int nl, const Leaf& L, double* area, double* Zg, long long ldz, int* status, int* unsure) {
     constexpr int s = W / 2;
     const int lane = threadIdx.x & 31;
     const Lanes<W> g{lane & (W - 1)};
@@ -498,7 +511,7 @@ __device__ void warp_level(int r0, int nl, const Leaf& L, double* area, double* 
     const long long ldd = last ? ldz : kLd;
     const int a = r0 + (lane & ~(W - 1));
     const int b = a + s < nl ? min(a + W, nl) : a;      // b == a: no second child
-    leaf_merge(g, a, s, b, L, Zc, U, nullptr, nullptr, status);
+    leaf_merge(g, a, s, b, L, Zc, U, nullptr, nullptr, status, unsure);
     if constexpr (W <= 8) {
         // one lane per column of the result
         const int nn = b - a, j = g.t;
@@ -541,7 +554,7 @@ __device__ void warp_level(int r0, int nl, const Leaf& L, double* area, double* 
 // the merges of 2 s = 512 / (512 / T) rows: T threads each
 template <int T>
 __device__ void block_level(int s, int nl, const Leaf& L, double* area, double* Zg, long long ldz, double* red,
-                            unsigned* words, int* status) {
+                            unsigned* words, int* status, int* unsure) {
     const int tid = threadIdx.x, mi = tid / T, a = 2 * s * mi;
     const Threads<T> g{tid % T};
     const double* Zc = area + child_off(s);
@@ -550,7 +563,7 @@ __device__ void block_level(int s, int nl, const Leaf& L, double* area, double* 
     double* out = last ? Zg : area + child_off(2 * s);
     const long long ldd = last ? ldz : kLd;
     const int b = a + s < nl ? min(a + 2 * s, nl) : a;
-    leaf_merge(g, a, s, b, L, Zc, U, red + 16 * mi, words + 4 * mi, status);
+    leaf_merge(g, a, s, b, L, Zc, U, red + 16 * mi, words + 4 * mi, status, unsure);
     const int nn = b - a;
     if (nn > 0) {
         const MergeSize m = merge_size(L.cnt + a, nn, s);
@@ -573,7 +586,8 @@ constexpr size_t kLeafSmem = sizeof(double) * (kAreaEnd + kLeafDoubles + 32 + 4)
 // Rows c0 .. c0 + nl - 1 (nl <= 128) of a tridiagonal matrix of order n: eigenvalues
 // (ascending) to D, eigenvectors to the diagonal block of Z (leading dimension n); the rest
 // of those columns of Z is set to zero.  512 threads; sm: kLeafSmem bytes.
-__device__ void dc_leaf(int c0, int nl, int n, double* D, const double* E, double* Z, double* sm, int* status) {
+__device__ void dc_leaf(int c0, int nl, int n, double* D, const double* E, double* Z, double* sm, int* status,
+                        int* unsure = nullptr) {
     const int tid = threadIdx.x, warp = tid >> 5;
     double* area = sm;
     const Leaf L = leaf_at(sm + kAreaEnd);
@@ -605,16 +619,16 @@ __device__ void dc_leaf(int c0, int nl, int n, double* D, const double* E, doubl
         if (nl == 1) {
             if (tid == 0) Zg[0] = 1.0;
         } else {
-            warp_level<2>(r0, nl, L, area, Zg, n, status);
-            if (nl > 2) warp_level<4>(r0, nl, L, area, Zg, n, status);
-            if (nl > 4) warp_level<8>(r0, nl, L, area, Zg, n, status);
-            if (nl > 8) warp_level<16>(r0, nl, L, area, Zg, n, status);
-            if (nl > 16) warp_level<32>(r0, nl, L, area, Zg, n, status);
+            warp_level<2>(r0, nl, L, area, Zg, n, status, unsure);
+            if (nl > 2) warp_level<4>(r0, nl, L, area, Zg, n, status, unsure);
+            if (nl > 4) warp_level<8>(r0, nl, L, area, Zg, n, status, unsure);
+            if (nl > 8) warp_level<16>(r0, nl, L, area, Zg, n, status, unsure);
+            if (nl > 16) warp_level<32>(r0, nl, L, area, Zg, n, status, unsure);
         }
     }
     __syncthreads();
-    if (nl > 32) block_level<256>(32, nl, L, area, Zg, n, red, words, status);
-    if (nl > 64) block_level<512>(64, nl, L, area, Zg, n, red, words, status);
+    if (nl > 32) block_level<256>(32, nl, L, area, Zg, n, red, words, status, unsure);
+    if (nl > 64) block_level<512>(64, nl, L, area, Zg, n, red, words, status, unsure);
     if (tid < nl) D[c0 + tid] = L.D[tid];
 }
 

@@ -97,19 +97,22 @@ static_assert(kPanelThreads == kBtThreads && kPanelMax <= kMaxN, "the back-trans
 
 __global__ void __launch_bounds__(kPanelThreads) k_syev_panel(const SyevSector* __restrict__ secs, double* __restrict__ eigbuf,
                                                              double* __restrict__ evals, double* __restrict__ wsd,
+                                                             const int* __restrict__ unsure, const double* from,
                                                              int* status) {
     extern __shared__ __align__(16) double sm[];
+    if (unsure && *unsure == 0) return;
     const SyevSector sec = secs[blockIdx.x];
     const int n = sec.n;
     const int tid = threadIdx.x, T = blockDim.x;
     double* A = eigbuf + sec.a_off;
     double* ev = evals + sec.e_off;
+    if (!from) from = A;
     const long long sq = (long long)n * n;
     {
         // a block holding NaN or Inf is reported and left undiagonalised (its eigenvalues
         // become NaN)
         bool bad = false;
-        for (long long e = tid; e < sq; e += T) bad |= !isfinite(A[e]);
+        for (long long e = tid; e < sq; e += T) bad |= !isfinite(from[e]);
         if (__syncthreads_or(bad)) {
             if (tid == 0) atomicOr(status, NRG_DEV_NONFINITE);
             for (int i = tid; i < n; i += T) ev[i] = __longlong_as_double(0x7ff8000000000000LL);
@@ -117,7 +120,7 @@ __global__ void __launch_bounds__(kPanelThreads) k_syev_panel(const SyevSector* 
         }
     }
     if (n == 1) {
-        if (tid == 0) { ev[0] = A[0]; A[0] = 1.0; }
+        if (tid == 0) { ev[0] = from[0]; A[0] = 1.0; }
         return;
     }
     double* W = wsd + sec.w_off;
@@ -133,7 +136,7 @@ __global__ void __launch_bounds__(kPanelThreads) k_syev_panel(const SyevSector* 
     const Scratch S = scratch_smem(Dm, kPanelMax);
 
     // ---- 1. tridiagonalisation in shared memory ----
-    for (long long e = tid; e < sq; e += T) As[e] = A[e];
+    for (long long e = tid; e < sq; e += T) As[e] = from[e];
     __syncthreads();
     tridiagonalise(As, n, n, Dd, Ee, TAU, vs, ps, red);
     for (long long e = tid; e < sq; e += T) A[e] = As[e];
@@ -1280,11 +1283,11 @@ int panel_merges(nrg_context* ctx, const std::vector<LSec>& secs, const LSec* ds
 
 }  // namespace nrg
 
-int launch_syev_panel(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* d_status,
-                      cudaStream_t st) {
+int launch_syev_panel(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, const int* unsure,
+                      const double* from, int* d_status, cudaStream_t st) {
     if (nsec == 0) return NRG_OK;
     NRG_TRY(nrg::raise_smem_limit((const void*)k_syev_panel, kPanelSmem));
-    k_syev_panel<<<nsec, kPanelThreads, kPanelSmem, st>>>(d_secs, eigbuf, evals, wsd, d_status);
+    k_syev_panel<<<nsec, kPanelThreads, kPanelSmem, st>>>(d_secs, eigbuf, evals, wsd, unsure, from, d_status);
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
 }

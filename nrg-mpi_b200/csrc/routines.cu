@@ -408,10 +408,10 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
         const cudaStream_t st = fork_small ? ctx->aux : ctx->stream;
         int* d_status = ctx->d_status.as<int>();
         if (solver == EigSolver::Panel) {
-            rl = launch_syev_panel(small, nsec - nlarge, d_V, d_E, bwd.as<double>(), d_status, st);
+            rl = launch_syev_panel(small, nsec - nlarge, d_V, d_E, bwd.as<double>(), nullptr, nullptr, d_status, st);
             ctx->launches++;
         } else {
-            rl = launch_syev(small, nsec - nlarge, d_V, d_E, bwd.as<double>(), bwi.as<int>(), d_status, st);
+            rl = launch_syev(small, nsec - nlarge, d_V, d_E, bwd.as<double>(), nullptr, d_status, st);
             ctx->launches += 2;
         }
     }

@@ -4,13 +4,15 @@ index of its entry of largest magnitude and whether that entry is negative, as
 nrg_diagonalization returned them before the reduction of the device-resident runs was
 replaced; the solver of those runs returns columns 4 and 849 of the first one (and others) with
 the opposite sign."""
+import ctypes
 import math
 import os
 
 import numpy as np
 import pytest
+import torch
 
-from nrg_b200 import model, prepare_basis
+from nrg_b200 import load_library, model, prepare_basis
 
 pytestmark = pytest.mark.gpu
 
@@ -36,6 +38,28 @@ def test_sector_signs(n, seed, ctx_factory):
     c0 = int(q[3]) - 1
     V = V[c0:c0 + n * n].reshape((n, n), order="F")
     with np.load(GOLDEN) as g:
+        entry = g[f"entry_{n}_{seed}"]
+        negative = np.unpackbits(g[f"negative_{n}_{seed}"], count=n).astype(bool)
+    assert np.array_equal(np.nonzero((V[entry, np.arange(n)] < 0) != negative)[0], [])
+
+
+@pytest.mark.parametrize("n,seed", [(17, 3), (64, 2), (100, 1), (128, 0), (128, 2456)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_block_signs(n, seed, in_place):
+    """The same of nrg_block_eigh_noalloc (golden/block_signs.npz); the faster solver alone
+    returns column 6 of the last block with the opposite sign."""
+    rng = np.random.default_rng(10000 + seed)
+    H = rng.standard_normal((n, n)) / math.sqrt(n)
+    H = (H + H.T) / 2 + np.diag(np.sort(7.0 * rng.random(n) ** 0.45))
+    fn = load_library().nrg_block_eigh_noalloc
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    h = torch.from_numpy(H).cuda()
+    E = torch.zeros(n, dtype=torch.float64, device="cuda")
+    V = h if in_place else torch.zeros_like(h)
+    assert fn(h.data_ptr(), n, E.data_ptr(), V.data_ptr(), None) == 0
+    V = V.cpu().numpy().T
+    assert np.max(np.abs(H @ V - V * E.cpu().numpy())) < 20 * n * np.finfo(np.float64).eps * np.linalg.norm(H, 2)
+    with np.load(os.path.join(os.path.dirname(GOLDEN), "block_signs.npz")) as g:
         entry = g[f"entry_{n}_{seed}"]
         negative = np.unpackbits(g[f"negative_{n}_{seed}"], count=n).astype(bool)
     assert np.array_equal(np.nonzero((V[entry, np.arange(n)] < 0) != negative)[0], [])
