@@ -33,6 +33,16 @@ __device__ double block_max(double v, double* red) {
     return s;
 }
 
+// v, or zero with the status flag set where v is not finite.  Every diagonal entry and merged
+// value of the divide and conquer passes here: ranks among them are used as indexes, and with a
+// NaN (a norm that overflowed in the reduction, a wait that ran out) two entries would share a
+// rank and leave another unwritten.
+__device__ __forceinline__ double finite_value(double v, int* status) {
+    if (isfinite(v)) return v;
+    atomicOr(status, NRG_DEV_NONFINITE);
+    return 0.0;
+}
+
 // scratch arrays of one sector, each of length n, indexed by absolute row
 struct Scratch {
     double *z, *ds, *zs, *dd, *zz, *tau, *zh, *vals, *rc, *rs;

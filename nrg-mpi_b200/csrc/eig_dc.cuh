@@ -456,7 +456,7 @@ __device__ void leaf_merge(const G& g, int a, int s, int b, const Leaf& L, const
     // the merged values, nondeflated roots first, and their places in ascending order (ties
     // keep list order)
     double* vals = L.vals + a;
-    for (int e = t; e < nn; e += T) vals[e] = e < K ? dd[org[e]] + tau[e] : ds[df[e - K]];
+    for (int e = t; e < nn; e += T) vals[e] = finite_value(e < K ? dd[org[e]] + tau[e] : ds[df[e - K]], status);
     if (nrot)
         for (int q = t; q < nn - K; q += T) {
             U[perm[df[q]] * kLd + a + K + q] = 1.0;
@@ -600,9 +600,10 @@ __device__ void dc_leaf(int c0, int nl, int n, double* D, const double* E, doubl
         if (tid < nl) {
             const int i = c0 + tid;
             dv = D[i];
-            ev = E[i];
+            ev = finite_value(E[i], status);
             if (i > 0) dv -= fabs(E[i - 1]);
             if (i < n - 1) dv -= fabs(ev);
+            dv = finite_value(dv, status);
         }
         L.D[tid] = dv;
         L.E[tid] = ev;

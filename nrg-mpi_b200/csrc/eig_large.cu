@@ -241,7 +241,8 @@ __device__ int block_scan(int v, bool maximum, int* red) {
 // negligible ones; chain starts in `nd`'s tail are not needed: rotation r continues the
 // one before when it shares its entry.
 __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(const LSec* __restrict__ secs, const Merge* __restrict__ ms,
-                                                          long long z_off, double* eigbuf, double* wsd, int* wsi) {
+                                                          long long z_off, double* eigbuf, double* wsd, int* wsi,
+                                                          int* status) {
     extern __shared__ __align__(16) double psm[];
     __shared__ double red[32];
     __shared__ int ired[32];
@@ -376,7 +377,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(const LSec* __restrict
     const int K = L.S.mk[a];
     for (int q = t; q < nn - K; q += kPrepThreads) {
         const int r = df[q];
-        L.S.vals[a + K + q] = ds[r];
+        L.S.vals[a + K + q] = finite_value(ds[r], status);
         df[q] = perm[r];
     }
 }
@@ -415,7 +416,7 @@ __global__ void __launch_bounds__(TPB) k_dc_items(const LSec* __restrict__ secs,
         if (e < K) {
             leaf_root(g, lane, K, dd, zz, rho, e, L.S.org + a + e, L.S.tau + a + e, status);
             __syncwarp();
-            if (lane == 0) L.S.vals[a + e] = dd[org[e]] + tau[e];
+            if (lane == 0) L.S.vals[a + e] = finite_value(dd[org[e]] + tau[e], status);
         }
     } else if constexpr (PHASE == 2) {
         if (alone) return;
@@ -1023,7 +1024,7 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         const Merge* dms = bmrg.as<Merge>();
         int* d_status = ctx->d_status.as<int>();
         const size_t psm = std::min(kPrepSmem, 4 * sizeof(double) * (size_t)widest);
-        k_dc_prep<<<nm, kPrepThreads, psm, st>>>(dsec, dms, z_in, d_V, wsd, wsi);
+        k_dc_prep<<<nm, kPrepThreads, psm, st>>>(dsec, dms, z_in, d_V, wsd, wsi, d_status);
         k_dc_items<1><<<blk, TPB, 0, st>>>(dsec, dms, nm, z_in, z_out, d_V, wsd, wsi, d_status);
         k_dc_items<2><<<blk, TPB, 0, st>>>(dsec, dms, nm, z_in, z_out, d_V, wsd, wsi, d_status);
         k_dc_items<3><<<blk, TPB, 0, st>>>(dsec, dms, nm, z_in, z_out, d_V, wsd, wsi, d_status);

@@ -426,13 +426,13 @@ __device__ void merge_ucols(int t, int T, int a, int n, Scratch S, double* U, R 
 }
 
 // the merged values in list order: nondeflated roots, then the deflated values
-__device__ void merge_vals(int t, int T, int a, int b, Scratch S) {
+__device__ void merge_vals(int t, int T, int a, int b, Scratch S, int* status) {
     const int K = S.mk[a], nn = b - a;
     const double* dd = S.dd + a;
     const int* org = S.org + a;
     const double* tau = S.tau + a;
     for (int e = t; e < nn; e += T)
-        S.vals[a + e] = e < K ? dd[org[e]] + tau[e] : S.ds[a + S.df[a + (e - K)]];
+        S.vals[a + e] = finite_value(e < K ? dd[org[e]] + tau[e] : S.ds[a + S.df[a + (e - K)]], status);
 }
 
 // final ascending order: nondeflated roots (list position j) then deflated values
@@ -486,7 +486,7 @@ __device__ void dc_merge(G g, int a, int mid, int b, int n, double* Z, double* D
     merge_zhat(t / kMergeLanes, T / kMergeLanes, a, mid, E, S, gl);
     g.sync();
     merge_ucols(t / kMergeLanes, T / kMergeLanes, a, n, S, U, gl);
-    merge_vals(t, T, a, b, S);
+    merge_vals(t, T, a, b, S, status);
     g.sync();
     merge_rank(t, T, a, b, S);
     g.sync();

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kPanelThreads) k_syev_panel(const SyevSector* 
         double dv = Dd[i];
         if (i > 0) dv -= fabs(Ee[i - 1]);
         if (i < n - 1) dv -= fabs(Ee[i]);
-        Dm[i] = dv;
+        Dm[i] = finite_value(dv, status);
     }
     __syncthreads();
     const int warp = tid >> 5, lane = tid & 31, nwarps = T >> 5;
@@ -965,7 +965,7 @@ __global__ void __launch_bounds__(512) k_dc_low(const LSec* __restrict__ secs, i
         double dv = L.D[i];
         if (i > 0) dv -= fabs(L.E[i - 1]);
         if (i < n - 1) dv -= fabs(L.E[i]);
-        Dl[i - c0] = dv;
+        Dl[i - c0] = finite_value(dv, status);
     }
     __syncthreads();
     const int warp = tid >> 5, lane = tid & 31, nwarps = T >> 5;
@@ -1038,7 +1038,7 @@ __global__ void __launch_bounds__(TPB) k_dc_phase(const LSec* __restrict__ secs,
                 for (int j = t >> 5; j < K; j += T >> 5)
                     for (int i = K + (t & 31); i < nn; i += 32) L.U[(size_t)(m.a + i) + (size_t)(m.a + j) * L.n] = 0.0;
             }
-            merge_vals(t, T, m.a, m.b, L.S);
+            merge_vals(t, T, m.a, m.b, L.S, status);
             break;
         case 4: {
             merge_rank(t, T, m.a, m.b, L.S);
