@@ -34,6 +34,14 @@ enum : int {
     NRG_DEV_TIMEOUT = 16,        // a bounded wait between blocks expired
 };
 
+// the status a call returns for these flags.  A wait that ran out comes first: what else is set
+// may be its consequence.
+inline int device_status_code(int flags) {
+    if (flags == NRG_DEV_OK) return NRG_OK;
+    if (flags & NRG_DEV_TIMEOUT) return NRG_ERR_TIMEOUT;
+    return (flags & (NRG_DEV_SECULAR | NRG_DEV_NONFINITE)) ? NRG_ERR_NUMERIC : NRG_ERR_INVALID;
+}
+
 // --------------------------------------------------------------------------------------
 // eigensolver work description (one entry per symmetry sector)
 // --------------------------------------------------------------------------------------

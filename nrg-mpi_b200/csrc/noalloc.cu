@@ -155,7 +155,7 @@ extern "C" int nrg_block_eigh_noalloc(const double* H, int32_t n, double* eigenv
     NRG_CUDA_TRY(cudaStreamSynchronize(st));
     if (flags != 0) {
         nrg_set_error_message("nrg_block_eigh_noalloc: device status flags 0x%x", flags);
-        return NRG_ERR_NUMERIC;
+        return device_status_code(flags);
     }
     return NRG_OK;
 }

@@ -294,8 +294,8 @@ int check_device_status(nrg_context* ctx) {
     if (st != 0) {
         NRG_CUDA_TRY(cudaMemsetAsync(ctx->d_status.p, 0, sizeof(int), ctx->stream));
         nrg_set_error_message("device status flags 0x%x (1: index out of range, 4: secular root, 8: NaN or Inf "
-                              "in a block)", st);
-        return (st & (NRG_DEV_SECULAR | NRG_DEV_NONFINITE)) ? NRG_ERR_NUMERIC : NRG_ERR_INVALID;
+                              "in a block, 16: a bounded wait expired)", st);
+        return device_status_code(st);
     }
     return NRG_OK;
 }
