@@ -825,7 +825,7 @@ namespace nrg {
 // ---------------------------------------------------------------------------------
 // host orchestration
 // ---------------------------------------------------------------------------------
-// NRG_TRI_CLUSTER=0 takes the multi-kernel tridiagonalisation for every sector of order > 128
+// NRG_TRI_CLUSTER=0 (a test aid) takes the multi-kernel tridiagonalisation for every sector of order > 128
 static bool tri_multi_kernel() {
     static const bool multi = [] {
         const char* e = getenv("NRG_TRI_CLUSTER");
@@ -913,7 +913,7 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
             if (c > 0) streamed.push_back(TriItem{A, vec, vec + n, vec + 2 * n, n, n, c, P});
             items.push_back(TriItem{A + c + (long long)c * n, vec + c, vec + n + c, vec + 2 * n + c, n - c, n, 0});
         }
-        NRG_TRY(tri_stream(ctx, streamed, tri_wide_clusters() ? 16 : 8, ctx->scratch.b[slot_base == 24 ? 48 : 49]));
+        NRG_TRY(tri_stream(ctx, streamed, ctx->scratch.b[slot_base == 24 ? 48 : 49]));
         NRG_TRY(tri_resident(ctx, items, ctx->scratch.b[slot_base == 24 ? 46 : 47]));
     }
     const bool clustered = nbig == 0;

@@ -35,7 +35,9 @@
 #include "internal.hpp"
 
 #include <algorithm>
+#include <array>
 #include <atomic>
+#include <cstdlib>
 
 namespace {
 
@@ -1118,8 +1120,13 @@ int launch_clusters(nrg_context* ctx, const TriTask* d_tasks, int blocks, size_t
 namespace nrg {
 
 // clusters of 16 blocks are beyond the portable size: where the device cannot place one,
-// the plans of 8 blocks are the largest
+// the plans of 8 blocks are the largest (NRG_TRI_CLUSTER=8 leaves 16 out: a test aid)
 int tri_resident_max() {
+    static const bool narrow = [] {
+        const char* e = getenv("NRG_TRI_CLUSTER");
+        return e && e[0] == '8' && e[1] == 0;
+    }();
+    if (narrow) return kPlanMax[kPlans - 2];
     static std::atomic<int> known[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kPlanMax[kPlans - 2];
@@ -1139,19 +1146,22 @@ int tri_resident_max() {
     return m;
 }
 
-bool tri_wide_clusters() { return tri_resident_max() == kPlanMax[kPlans - 1]; }
+// blocks of a streaming cluster: what fits in the shared memory of 8 is a little less than of 16
+static int stream_cluster() { return tri_resident_max() == kPlanMax[kPlans - 1] ? 16 : 8; }
 
 int tri_stream_max() {
-    static const int m = [] {
-        int n = 2;
-        while (8LL * StreamLayout(n + 1, 16, 1).doubles(16) <= kSmemMax) ++n;
-        return n;
+    static const std::array<int, 2> most = [] {
+        std::array<int, 2> m = {2, 2};
+        for (int i = 0; i < 2; ++i)
+            while (8LL * StreamLayout(m[i] + 1, 8 << i, 1).doubles(8 << i) <= kSmemMax) ++m[i];
+        return m;
     }();
-    return m;
+    return most[stream_cluster() / 16];
 }
 
-int tri_stream(nrg_context* ctx, const std::vector<TriItem>& items, int CL, DevBuf& buf) {
+int tri_stream(nrg_context* ctx, const std::vector<TriItem>& items, DevBuf& buf) {
     if (items.empty()) return NRG_OK;
+    const int CL = stream_cluster();
     std::vector<StreamTask> tasks;
     size_t smem = 0;
     for (const TriItem& it : items) {

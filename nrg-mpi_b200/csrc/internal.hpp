@@ -309,8 +309,8 @@ constexpr int kLargeSector = 128;
 // tridiagonalisation (eig_tri.cu) on ctx->stream: D, E, tau and the reflectors (below the
 // subdiagonal of A) of every item.  tri_resident: the matrix on chip, orders 2 ..
 // tri_resident_max().  tri_stream: the first `stop` columns of a larger one (up to
-// tri_stream_max(), lda = n) by clusters of CL = 8 or 16 blocks; the trailing block is left
-// updated for tri_resident.
+// tri_stream_max(), lda = n) by clusters of 16 blocks, or 8 where the device cannot place
+// those; the trailing block is left updated for tri_resident.
 struct TriItem {
     double* A;             // full symmetric storage, leading dimension lda
     double *D, *E, *TAU;
@@ -318,10 +318,9 @@ struct TriItem {
     double* P = nullptr;   // tri_stream: workspace of n ((n + 16) & ~15) doubles, 128-byte aligned
 };
 int tri_resident_max();
-bool tri_wide_clusters();   // clusters of 16 blocks can be placed
 int tri_resident(nrg_context* ctx, const std::vector<TriItem>& items, DevBuf& tasks);
 int tri_stream_max();
-int tri_stream(nrg_context* ctx, const std::vector<TriItem>& items, int CL, DevBuf& tasks);
+int tri_stream(nrg_context* ctx, const std::vector<TriItem>& items, DevBuf& tasks);
 
 // ---- kernels (kernels.cu) ------------------------------------------------------------
 int run_assemble(nrg_context* ctx, int iteration, const Sectors& S, const SyevSector* d_secs,
