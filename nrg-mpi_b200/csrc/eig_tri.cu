@@ -24,7 +24,9 @@
 // the receiver's mbarrier by byte count; no fence that would wait for the reflectors'
 // global stores).  Two exchange buffers suffice: a block sends step k + 2 only after it
 // has received all of step k + 1, which every block sends after its last read of step k's
-// buffer; a block whose columns are done leaves the loop.
+// buffer; a block whose columns are done leaves the loop.  Nothing is sent to a block that
+// will not wait for it: st.async may still be in flight when its sender has passed a cluster
+// barrier, so only a receiver's wait shows that it is done and the receiver may leave.
 //
 // Against the panel kernel (eig_large.cu), which streams the trailing matrix from L2 and
 // crosses two cluster barriers and about eight block barriers per column: 1.5..2.4 us per
@@ -266,6 +268,12 @@ __device__ __forceinline__ void tri_norm(const TriTask& t, double* sm, int k) {
     }
 }
 
+// whether block r of the group is in the loop at step k + 1, and so waits for what step k sends
+template <class P>
+__device__ __forceinline__ bool awaits(int r, int k, int n) {
+    return ((r - (k + 2)) & (P::CL - 1)) <= n - 1 - (k + 2);   // it has a column from k + 2 on
+}
+
 // the steps of the ninth warp
 template <class P>
 __device__ __forceinline__ void tri_norm_steps(const TriTask& t, double* sm, unsigned base) {
@@ -278,7 +286,7 @@ __device__ __forceinline__ void tri_norm_steps(const TriTask& t, double* sm, uns
         tri_norm<P>(t, sm, k);
         step_sync();
         if (sc[kScale] != 1.0) step_sync();
-        if (P::CL > 1 && k < n - 2 && lane < P::CL) {
+        if (P::CL > 1 && k < n - 2 && lane < P::CL && awaits<P>(lane, k, n)) {
             // the block's part of u.y
             const int nb = (k + 1) & 1;
             double s = 0.0;
@@ -478,7 +486,7 @@ __device__ __forceinline__ void tri_steps(const TriTask& t, double* sm, double (
                 constexpr int kParts = (P::kCols + 31) / 32;
                 for (int e = warp; e < CL * kParts; e += kTriWarps) {
                     const int r = e % CL, m = 32 * (e / CL) + lane;
-                    if (m < cnt && rank + CL * m >= rk) {
+                    if (m < cnt && rank + CL * m >= rk && awaits<P>(r, k, n)) {
                         double y = part[m];
 #pragma unroll
                         for (int g = 1; g < G; ++g) y += part[g * P::kCols + m];
@@ -547,7 +555,7 @@ __global__ void __launch_bounds__(kTriThreads, 1) k_tri_res(const TriTask* __res
     else ran = false;
     __syncwarp();
     if (!ran) asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
-    // no block leaves while another may still write its shared memory
+    // the blocks leave together (every message to one of them has been waited for)
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
@@ -1056,7 +1064,8 @@ __global__ void __launch_bounds__(kTriThreads, 1) k_tri_stream(const StreamTask*
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kNormRegs));
         if (warp == kTriWarps) stream_norm_steps<CL>(t, sm, to0);
     }
-    // no block leaves while another may still write its shared memory
+    // the blocks leave together: every message to one of them has been waited for, the last of
+    // them at the step that only completes the last update
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
