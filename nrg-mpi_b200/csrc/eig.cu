@@ -22,6 +22,7 @@ constexpr int kThreads = kLeafThreads;
 static_assert(kBtSmem <= kLeafSmem, "the back-transformation reuses the divide and conquer's shared memory");
 static_assert(kThreads == kBtThreads, "the back-transformation's block");
 
+template <bool MARK>
 __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict__ secs,
                                                     double* __restrict__ eigbuf,
                                                     double* __restrict__ evals,
@@ -42,12 +43,12 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
         if (__syncthreads_or(bad)) {
             if (tid == 0) atomicOr(status, NRG_DEV_NONFINITE);
             for (int i = tid; i < n; i += T) ev[i] = __longlong_as_double(0x7ff8000000000000LL);
-            if (unsure && tid == 0) *unsure = 0;
+            if (MARK && tid == 0) *unsure = 0;
             return;
         }
     }
     if (n == 1) {
-        if (tid == 0) { ev[0] = A[0]; A[0] = 1.0; if (unsure) *unsure = 0; }
+        if (tid == 0) { ev[0] = A[0]; A[0] = 1.0; if (MARK) *unsure = 0; }
         return;
     }
     double* W = wsd + sec.w_off;
@@ -59,9 +60,9 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
 
     // ---- 2. divide and conquer on (Dd, Ee) -> eigenvalues in Dd, vectors in Z ----
     if (tid == 0) maybe = 0;
-    dc_leaf(0, n, n, Dd, Ee, Z, sm, status, unsure ? &maybe : nullptr);   // (a barrier before its first merge)
+    dc_leaf<MARK>(0, n, n, Dd, Ee, Z, sm, status, &maybe);   // (a barrier before its first merge)
     __syncthreads();
-    if (unsure) {
+    if (MARK) {
         const double gap = kUnsureGap * fmax(fabs(Dd[0]), fabs(Dd[n - 1]));
         for (int i = tid; i < n - 1; i += T)
             if (Dd[i + 1] - Dd[i] <= gap) maybe = 1;
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
     // ---- 3. back-transformation, straight to the output ----
     back_transform(A, n, TAU, Z, sm);
     for (int i = tid; i < n; i += T) ev[i] = Dd[i];
-    if (unsure && tid == 0) *unsure = maybe;   // (back_transform has barriers before this)
+    if (MARK && tid == 0) *unsure = maybe;   // (back_transform has barriers before this)
 }
 
 }  // namespace
@@ -78,8 +79,9 @@ __global__ void __launch_bounds__(kThreads) k_syev(const SyevSector* __restrict_
 int launch_syev(const SyevSector* d_secs, int nsec, double* eigbuf, double* evals, double* wsd, int* unsure, int* d_status, cudaStream_t st) {
     if (nsec == 0) return NRG_OK;
     NRG_TRY(launch_tri_small(d_secs, nsec, eigbuf, wsd, d_status, st));
-    NRG_TRY(nrg::raise_smem_limit((const void*)k_syev, kLeafSmem));
-    k_syev<<<nsec, kThreads, kLeafSmem, st>>>(d_secs, eigbuf, evals, wsd, unsure, d_status);
+    auto kernel = unsure ? k_syev<true> : k_syev<false>;
+    NRG_TRY(nrg::raise_smem_limit((const void*)kernel, kLeafSmem));
+    kernel<<<nsec, kThreads, kLeafSmem, st>>>(d_secs, eigbuf, evals, wsd, unsure, d_status);
     NRG_CUDA_TRY(cudaGetLastError());
     return NRG_OK;
 }

@@ -295,13 +295,13 @@ __device__ __forceinline__ MergeSize merge_size(const int* cnt, int nn, int n1) 
 // k, column a + j; rows ordered by child, not normalised: 1 / norm in rn) and the places of
 // the results.  b == a: no merge, but the barriers are taken.
 //
-// unsure (may be null): set when the merge decides close to its tolerance, or between values so
+// MARK: *unsure is set when the merge decides close to its tolerance, or between values so
 // close (relative to the largest) that their eigenvectors hang on the last bits.  Of blocks of
 // order 128 with random entries 1 in 3,000 decides otherwise than the panel solver; the z of the
 // two differ by 0.3% of the tolerance there, so a quarter is a wide margin: it marks 10% of
 // them, a factor of 8 would mark 60%.
 constexpr double kUnsure = 1.25, kUnsureGap = 1e-6;
-template <class G>
+template <bool MARK, class G>
 __device__ void leaf_merge(const G& g, int a, int s, int b, const Leaf& L, const double* Zc, double* U, double* red,
                            unsigned* words, int* status, int* unsure) {
     const int t = g.rank(), T = g.size();
@@ -341,7 +341,7 @@ __device__ void leaf_merge(const G& g, int a, int s, int b, const Leaf& L, const
     g.sync();
     // ---- deflation: negligible z, then close neighbours among the others ----
     const bool in = t < nn;
-    if (unsure && in) {
+    if (MARK && in) {
         const double zr = rho * fabs(zs[t]);
         if ((zr > tol / kUnsure && zr < tol * kUnsure) ||
             (t > 0 && ds[t] - ds[t - 1] <= kUnsureGap / (8.0 * kEps) * tol))
@@ -499,7 +499,7 @@ __device__ __forceinline__ void leaf_deflated(int t, int T, int a, int s, int nn
 }
 
 // the levels of one warp's 32 rows: merges of W = 2 s rows, 32 / W at a time
-template <int W>
+template <int W, bool MARK>
 __device__ void warp_level(int r0, int nl, const Leaf& L, double* area, double* Zg, long long ldz, int* status, int* unsure) {
     constexpr int s = W / 2;
     const int lane = threadIdx.x & 31;
@@ -511,7 +511,7 @@ __device__ void warp_level(int r0, int nl, const Leaf& L, double* area, double* 
     const long long ldd = last ? ldz : kLd;
     const int a = r0 + (lane & ~(W - 1));
     const int b = a + s < nl ? min(a + W, nl) : a;      // b == a: no second child
-    leaf_merge(g, a, s, b, L, Zc, U, nullptr, nullptr, status, unsure);
+    leaf_merge<MARK>(g, a, s, b, L, Zc, U, nullptr, nullptr, status, unsure);
     if constexpr (W <= 8) {
         // one lane per column of the result
         const int nn = b - a, j = g.t;
@@ -552,7 +552,7 @@ __device__ void warp_level(int r0, int nl, const Leaf& L, double* area, double* 
 }
 
 // the merges of 2 s = 512 / (512 / T) rows: T threads each
-template <int T>
+template <int T, bool MARK>
 __device__ void block_level(int s, int nl, const Leaf& L, double* area, double* Zg, long long ldz, double* red,
                             unsigned* words, int* status, int* unsure) {
     const int tid = threadIdx.x, mi = tid / T, a = 2 * s * mi;
@@ -563,7 +563,7 @@ __device__ void block_level(int s, int nl, const Leaf& L, double* area, double* 
     double* out = last ? Zg : area + child_off(2 * s);
     const long long ldd = last ? ldz : kLd;
     const int b = a + s < nl ? min(a + 2 * s, nl) : a;
-    leaf_merge(g, a, s, b, L, Zc, U, red + 16 * mi, words + 4 * mi, status, unsure);
+    leaf_merge<MARK>(g, a, s, b, L, Zc, U, red + 16 * mi, words + 4 * mi, status, unsure);
     const int nn = b - a;
     if (nn > 0) {
         const MergeSize m = merge_size(L.cnt + a, nn, s);
@@ -586,6 +586,7 @@ constexpr size_t kLeafSmem = sizeof(double) * (kAreaEnd + kLeafDoubles + 32 + 4)
 // Rows c0 .. c0 + nl - 1 (nl <= 128) of a tridiagonal matrix of order n: eigenvalues
 // (ascending) to D, eigenvectors to the diagonal block of Z (leading dimension n); the rest
 // of those columns of Z is set to zero.  512 threads; sm: kLeafSmem bytes.
+template <bool MARK>
 __device__ void dc_leaf(int c0, int nl, int n, double* D, const double* E, double* Z, double* sm, int* status,
                         int* unsure = nullptr) {
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -620,16 +621,16 @@ __device__ void dc_leaf(int c0, int nl, int n, double* D, const double* E, doubl
         if (nl == 1) {
             if (tid == 0) Zg[0] = 1.0;
         } else {
-            warp_level<2>(r0, nl, L, area, Zg, n, status, unsure);
-            if (nl > 2) warp_level<4>(r0, nl, L, area, Zg, n, status, unsure);
-            if (nl > 4) warp_level<8>(r0, nl, L, area, Zg, n, status, unsure);
-            if (nl > 8) warp_level<16>(r0, nl, L, area, Zg, n, status, unsure);
-            if (nl > 16) warp_level<32>(r0, nl, L, area, Zg, n, status, unsure);
+            warp_level<2, MARK>(r0, nl, L, area, Zg, n, status, unsure);
+            if (nl > 2) warp_level<4, MARK>(r0, nl, L, area, Zg, n, status, unsure);
+            if (nl > 4) warp_level<8, MARK>(r0, nl, L, area, Zg, n, status, unsure);
+            if (nl > 8) warp_level<16, MARK>(r0, nl, L, area, Zg, n, status, unsure);
+            if (nl > 16) warp_level<32, MARK>(r0, nl, L, area, Zg, n, status, unsure);
         }
     }
     __syncthreads();
-    if (nl > 32) block_level<256>(32, nl, L, area, Zg, n, red, words, status, unsure);
-    if (nl > 64) block_level<512>(64, nl, L, area, Zg, n, red, words, status, unsure);
+    if (nl > 32) block_level<256, MARK>(32, nl, L, area, Zg, n, red, words, status, unsure);
+    if (nl > 64) block_level<512, MARK>(64, nl, L, area, Zg, n, red, words, status, unsure);
     if (tid < nl) D[c0 + tid] = L.D[tid];
 }
 

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kLeafThreads) k_dc_low(const LSec* __restrict_
     if (sidx >= nsec) return;
     LView L = lview(secs[sidx], eigbuf, wsd, wsi);
     const int c0 = bid * DC_LOW;
-    dc_leaf(c0, min(DC_LOW, L.n - c0), L.n, L.D, L.E, L.Z, sm, status);
+    dc_leaf<false>(c0, min(DC_LOW, L.n - c0), L.n, L.D, L.E, L.Z, sm, status);
 }
 
 // Merges beyond DC_LOW rows, all merges of one level at once, in five launches: poles and
