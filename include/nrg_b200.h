@@ -277,7 +277,7 @@ NRG_API int nrg_spike_cfs(nrg_context* ctx, int32_t iteration, const nrg_spike_i
  * column order.  H, eigenvalues and eigenvectors are caller-owned device arrays (H may
  * equal eigenvectors).  No context is needed: the call runs on the current device and on
  * `stream` (NULL = default stream), and returns after the stream has drained.
- * Its workspace is a static device array of about 417 KB, created on a device when the
+ * Its workspace is a static device array of about 396 KB, created on a device when the
  * library's device code is loaded there (with lazy module loading, the CUDA default, at
  * the first call on that device: a warm-up call during the caller's set-up keeps that
  * load out of later work) and held until the process exits.  The first call on a device

@@ -48,25 +48,15 @@ inline int device_status_code(int flags) {
 struct SyevSector {
     long long a_off;    // offset of the d x d block in the eigenvector buffer
     long long w_off;    // offset of the double workspace
-    long long i_off;    // offset of the int workspace
     long long e_off;    // offset of the eigenvalues (start_input - 1)
     int n;
     int pad;
 };
 
-// double workspace per sector of order n
-__host__ __device__ inline long long syev_ws_doubles(long long n) {
-    long long sq = n * n;
-    long long qt = sq > 64 * n ? sq : 64 * n;
-    return 2 * sq + qt + 16 * n + 64;
-}
-__host__ __device__ inline long long syev_ws_ints(long long n) { return 12 * n + 64; }
-
-// offset of D | E | tau (n doubles each) and the divide-and-conquer vectors in it
-__host__ __device__ inline long long syev_vec_off(long long n) {
-    const long long sq = n * n;
-    return 2 * sq + (sq > 64 * n ? sq : 64 * n);
-}
+// workspace of a sector of order n <= 128, in doubles: the eigenvectors of T, two more n x n
+// arrays for the panel solver's merges, then D | E | tau (n each)
+__host__ __device__ constexpr long long syev_vec_off(long long n) { return 3 * n * n; }
+__host__ __device__ constexpr long long syev_ws_doubles(long long n) { return syev_vec_off(n) + 3 * n; }
 
 // launch helpers implemented in the .cu files (return NRG status)
 int launch_tri_small(const SyevSector* d_secs, int nsec, double* eigbuf, double* wsd, int* d_status, cudaStream_t st);

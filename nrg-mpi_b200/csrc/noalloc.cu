@@ -12,18 +12,15 @@ namespace {
 
 // largest block order the static workspace covers
 constexpr long long kMaxN = NRG_NOALLOC_MAX_ORDER;
-constexpr long long kWsDoubles = 2 * kMaxN * kMaxN + (kMaxN * kMaxN > 64 * kMaxN ? kMaxN * kMaxN : 64 * kMaxN) +
-                                 16 * kMaxN + 64;
-constexpr long long kWsInts = 12 * kMaxN + 64;
-constexpr long long kIntsAsDoubles = (kWsInts + 1) / 2;
-// [0, 8): sector descriptor, [8, 16): status word, then the int and double workspaces
-constexpr long long kDescOff = 0, kStatusOff = 8, kIntOff = 16, kDblOff = kIntOff + kIntsAsDoubles;
-constexpr long long kTotalDoubles = kDblOff + kWsDoubles;
+// [0, 8): sector descriptor, [8, 16): status word and the mark of a close decision, then the
+// workspace
+constexpr long long kDescOff = 0, kStatusOff = 8, kDblOff = 16;
+constexpr long long kTotalDoubles = kDblOff + syev_ws_doubles(kMaxN);
 static_assert(sizeof(SyevSector) <= 8 * sizeof(double), "descriptor slot too small");
 
 }  // namespace
 
-// the workspace: one copy per device that loads the library (~417 KB), kept until exit
+// the workspace: one copy per device that loads the library (~396 KB), kept until exit
 static __device__ __align__(256) double g_noalloc_scratch[kTotalDoubles];
 
 namespace {
@@ -128,13 +125,12 @@ extern "C" int nrg_block_eigh_noalloc(const double* H, int32_t n, double* eigenv
     SyevSector sec;
     sec.a_off = 0;
     sec.w_off = 0;
-    sec.i_off = 0;
     sec.e_off = 0;
     sec.n = n;
     sec.pad = 0;
     SyevSector* d_sec = reinterpret_cast<SyevSector*>(base + kDescOff);
     int* d_status = reinterpret_cast<int*>(base + kStatusOff);
-    int* d_ints = reinterpret_cast<int*>(base + kIntOff);
+    int* d_unsure = d_status + 1;
     double* d_ws = base + kDblOff;
     // the workspace keeps the previous call's contents: the status word must start at zero;
     // the eigensolver writes every other workspace entry before reading it
@@ -148,8 +144,8 @@ extern "C" int nrg_block_eigh_noalloc(const double* H, int32_t n, double* eigenv
     double* kept = d_ws + (long long)n * n;   // in place: the block, where only the panel solver works
     if (eigenvectors == H)
         NRG_CUDA_TRY(cudaMemcpyAsync(kept, H, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st));
-    NRG_TRY(launch_syev(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_ints, d_status, st));
-    NRG_TRY(launch_syev_panel(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_ints, eigenvectors == H ? kept : H, d_status, st));
+    NRG_TRY(launch_syev(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, d_status, st));
+    NRG_TRY(launch_syev_panel(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, eigenvectors == H ? kept : H, d_status, st));
     int flags = 0;
     NRG_CUDA_TRY(cudaMemcpyAsync(&flags, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     NRG_CUDA_TRY(cudaStreamSynchronize(st));

@@ -316,7 +316,7 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
     std::vector<SyevSector> secs(nsec);
     std::vector<long long> colPrefix(nsec);
     std::vector<int> secStart(nsec);
-    long long wsd = 0, wsi = 0, cols = 0;
+    long long wsd = 0, cols = 0;
     int nlarge = 0;
     std::vector<SyevSector> large;
     for (int x = 0; x < nsec; ++x) {
@@ -326,16 +326,13 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
         q.a_off = S.ce[s];
         q.e_off = S.start[s];
         q.w_off = 0;
-        q.i_off = 0;
         q.pad = 0;
         if (q.n > kLargeSector) {
             large.push_back(q);
             ++nlarge;
         } else {
             q.w_off = wsd;
-            q.i_off = wsi;
             wsd += syev_ws_doubles(q.n);
-            wsi += syev_ws_ints(q.n);
         }
         colPrefix[x] = cols;
         cols += q.n;
@@ -345,13 +342,11 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
     DevBuf& bcol = ctx->scratch.b[1];
     DevBuf& bstart = ctx->scratch.b[2];
     DevBuf& bwd = ctx->scratch.b[3];
-    DevBuf& bwi = ctx->scratch.b[4];
     DevBuf& bmin = ctx->scratch.b[5];
     NRG_TRY(bsec.ensure(sizeof(SyevSector) * nsec));
     NRG_TRY(bcol.ensure(sizeof(long long) * nsec));
     NRG_TRY(bstart.ensure(sizeof(int) * nsec));
     NRG_TRY(bwd.ensure(sizeof(double) * (size_t)std::max(wsd, 1LL)));
-    NRG_TRY(bwi.ensure(sizeof(int) * (size_t)std::max(wsi, 1LL)));
     NRG_TRY(bmin.ensure(sizeof(double) * 2));
     NRG_TRY(h2d_async(ctx, bsec.p, secs.data(), sizeof(SyevSector) * nsec));
     NRG_TRY(h2d_async(ctx, bcol.p, colPrefix.data(), sizeof(long long) * nsec));
