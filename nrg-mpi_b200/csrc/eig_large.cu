@@ -835,7 +835,7 @@ static bool tri_multi_kernel() {
 }
 
 int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V, double* d_E, EigSolver solver,
-               int slot_base, cudaEvent_t evals_ready) {
+               const EigSlots& slots, cudaEvent_t evals_ready) {
     const bool panel = solver == EigSolver::Panel;
     const int ns = (int)in.size();
     if (ns == 0) return NRG_OK;
@@ -856,12 +856,12 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
         wi += lws_ints(in[s].n);
         maxn = std::max(maxn, in[s].n);
     }
-    DevBuf& bsec = ctx->scratch.b[slot_base];
-    DevBuf& bwd = ctx->scratch.b[slot_base + 1];
-    DevBuf& bwi = ctx->scratch.b[slot_base + 2];
-    DevBuf& bidx = ctx->scratch.b[slot_base + 3];
-    DevBuf& bmrg = ctx->scratch.b[slot_base + 4];
-    const int gslot = slot_base + 5;   // grouped GEMM problem lists (two slots)
+    DevBuf& bsec = ctx->scratch.b[slots.sectors];
+    DevBuf& bwd = ctx->scratch.b[slots.doubles];
+    DevBuf& bwi = ctx->scratch.b[slots.ints];
+    DevBuf& bidx = ctx->scratch.b[slots.columns];
+    DevBuf& bmrg = ctx->scratch.b[slots.merges];
+    const int gslot = slots.products;   // grouped GEMM problem lists
     NRG_TRY(bsec.ensure(sizeof(LSec) * ns));
     NRG_TRY(bwd.ensure(sizeof(double) * (size_t)wd));
     NRG_TRY(bwi.ensure(sizeof(int) * (size_t)wi));
@@ -913,8 +913,8 @@ int syev_large(nrg_context* ctx, const std::vector<SyevSector>& in, double* d_V,
             if (c > 0) streamed.push_back(TriItem{A, vec, vec + n, vec + 2 * n, n, n, c, P});
             items.push_back(TriItem{A + c + (long long)c * n, vec + c, vec + n + c, vec + 2 * n + c, n - c, n, 0});
         }
-        NRG_TRY(tri_stream(ctx, streamed, ctx->scratch.b[slot_base == 24 ? 48 : 49]));
-        NRG_TRY(tri_resident(ctx, items, ctx->scratch.b[slot_base == 24 ? 46 : 47]));
+        NRG_TRY(tri_stream(ctx, streamed, ctx->scratch.b[slots.streamed]));
+        NRG_TRY(tri_resident(ctx, items, ctx->scratch.b[slots.on_chip]));
     }
     const bool clustered = nbig == 0;
     if (ctx->profiling) {

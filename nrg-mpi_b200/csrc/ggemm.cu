@@ -31,14 +31,10 @@
 namespace nrg {
 namespace {
 
-// d (16 x 8) += a (16 x 8) b (8 x 8): lane l holds a(l / 4 + {0, 8}, l % 4 + {0, 4}), b(l % 4 + {0, 4},
-// l / 4) and d(l / 4 + {0, 8}, 2 (l % 4) + {0, 1}); 3-5% over twice m8n8k4 pairs
+// the 16 x 8 x 8 MMA on fragments held as [row half][k half]; 3-5% over twice m8n8k4 pairs
 __device__ __forceinline__ void dmma16(double (&d)[2][2], const double (&a)[2][2], const double (&b)[2]) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};\n"
-        : "+d"(d[0][0]), "+d"(d[0][1]), "+d"(d[1][0]), "+d"(d[1][1])
-        : "d"(a[0][0]), "d"(a[1][0]), "d"(a[0][1]), "d"(a[1][1]), "d"(b[0]), "d"(b[1]));
+    nrg::cta_dmma16(d[0][0], d[0][1], d[1][0], d[1][1], make_double2(a[0][0], a[1][0]), make_double2(a[0][1], a[1][1]),
+                    b[0], b[1]);
 }
 
 // (16 WM RM) x (8 WN RN) output tile of WM x WN warps with RM x RN MMA tiles each.  Every variant

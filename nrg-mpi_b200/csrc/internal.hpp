@@ -293,13 +293,20 @@ int launch_ggemm(nrg_context* ctx, std::vector<GemmProblem>& probs, int scratch_
 // version of the code to the next.
 enum class EigSolver { Device, Panel };
 
+// scratch slots of one syev_large call
+struct EigSlots {
+    int sectors, doubles, ints, columns, merges, products, on_chip, streamed;
+};
+constexpr EigSlots kEigSlots[2] = {{24, 25, 26, 27, 28, 29, 46, 48}, {31, 32, 33, 34, 35, 36, 47, 49}};
+
 // eigensolver for sectors of order > 128 across the whole GPU (eig_large.cu); the
 // descriptors use a_off / e_off / n only
-// (scratch slots slot_base .. slot_base + 6; on ctx->stream)
+// (on ctx->stream).  Two calls may be in flight on two streams of one context, with a slot set
+// each.
 // evals_ready (optional) is recorded on ctx->stream once the eigenvalues are in d_E,
 // before the back-transformation
 int syev_large(nrg_context* ctx, const std::vector<SyevSector>& secs, double* d_V, double* d_E, EigSolver solver,
-               int slot_base, cudaEvent_t evals_ready = nullptr);
+               const EigSlots& slots, cudaEvent_t evals_ready = nullptr);
 struct LSec;
 int panel_tridiagonal(nrg_context* ctx, const LSec* dsec, int ns, int maxn, double* d_V, double* wsd, int* wsi, bool* done);
 int panel_merges(nrg_context* ctx, const std::vector<LSec>& secs, const LSec* dsec, int maxn, double* d_V, double* wsd,

@@ -391,11 +391,11 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
         NRG_CUDA_TRY(cudaStreamWaitEvent(s1, ctx->ev_fork, 0));
         cudaStream_t caller = ctx->stream;
         ctx->stream = s1;
-        rl = syev_large(ctx, g1, d_V, d_E, solver, 24, early && !g1.empty() ? ctx->ev_evals_hi : nullptr);
+        rl = syev_large(ctx, g1, d_V, d_E, solver, kEigSlots[0], early && !g1.empty() ? ctx->ev_evals_hi : nullptr);
         ctx->stream = caller;
         NRG_CUDA_TRY(cudaEventRecord(ctx->ev_join_hi, s1));
     } else {
-        rl = syev_large(ctx, g1, d_V, d_E, solver, 24);
+        rl = syev_large(ctx, g1, d_V, d_E, solver, kEigSlots[0]);
     }
     if (fork_small) NRG_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
     if (nsec > nlarge && rl == NRG_OK) {
@@ -416,7 +416,7 @@ int diag_device(nrg_context* ctx, int iteration, Sectors& S, const double* d_Eol
         NRG_CUDA_TRY(cudaStreamWaitEvent(ctx->aux2, ctx->ev_fork, 0));
         cudaStream_t caller = ctx->stream;
         ctx->stream = ctx->aux2;
-        if (rl == NRG_OK) rl = syev_large(ctx, g2, d_V, d_E, solver, 31, early ? ctx->ev_evals2 : nullptr);
+        if (rl == NRG_OK) rl = syev_large(ctx, g2, d_V, d_E, solver, kEigSlots[1], early ? ctx->ev_evals2 : nullptr);
         ctx->stream = caller;
         NRG_CUDA_TRY(cudaEventRecord(ctx->ev_join2, ctx->aux2));
     }
