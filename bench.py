@@ -75,7 +75,8 @@ WORKLOAD_NAME = ("SIAM flat band Lambda=2.0 U=0.3 Gamma=0.03 eps_d=-0.15 N_keep=
                  "60 NRG iterations + backward RDM + T=0 CFS spectrum (1000 bins/decade)")
 SECOND = dict(U=0.2, Gamma=0.02, eps_d=-0.1, Lambda=2.0, n_keep=2048, n_iterations=60)
 METRIC = "NRG iterations/s (full sweep + RDM + CFS spectrum, FP64, eig err <= 1e-12)"
-# DRAM bytes per launch of the roofline kernel, from an ncu capture of this workload
+# DRAM bytes of the roofline kernels, from an ncu capture of the largest sector class's order (not of
+# this workload's own launches, whose sizes are mixed)
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "roofline_traffic.json")
 
 
@@ -390,11 +391,13 @@ def oracle_window(n_full, warmup=0):
 
 
 def roofline_traffic():
-    """DRAM bytes per launch pair of the roofline kernels (ncu), if captured."""
+    """DRAM bytes per launch pair of the roofline kernels (ncu), if captured, and of what."""
     try:
         with open(TRAFFIC_FILE) as f:
             t = json.load(f)
-        return float(t["bytes_per_launch"]), os.path.relpath(TRAFFIC_FILE, ROOT)
+        b, flops = float(t["bytes_per_launch"]), float(t["flops_per_launch"])
+        return b, {"file": os.path.relpath(TRAFFIC_FILE, ROOT), "workload": t["workload"], "flops_per_launch": flops,
+                   "bytes_per_flop": b / flops}
     except (OSError, ValueError, KeyError):
         return None, None
 
