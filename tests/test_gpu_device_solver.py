@@ -46,3 +46,53 @@ def test_sectors(env, orders):
                        capture_output=True, text=True, timeout=900)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
     assert r.stdout.count("passed") == len(orders)
+
+
+MIXED = """
+import math, sys
+sys.path[:0] = [{root!r}, {package!r}]
+import numpy as np, torch
+from nrg_b200 import Context, model, prepare_basis
+it, ka, kb = 8, 3500, 100
+n = ka + kb
+rng = np.random.default_rng(n)
+inp = model.siam(U=0.2, Gamma=0.02, eps_d=-0.1, Lambda=2.0, n_keep=64, n_iterations=20)
+ctx = Context(0)
+ctx.set_model(inp)
+rec = np.zeros((n, 5), dtype=np.int32)
+rec[:ka, 2], rec[ka:, :2], rec[ka:, 2] = np.arange(1, ka + 1), (1, 1), np.arange(1, kb + 1)
+E_old = np.concatenate([np.sort(7 * rng.random(ka)), np.sort(7 * rng.random(kb))])
+im = np.zeros((n, n, 2), order="F")
+im[:ka, ka:, 0] = rng.standard_normal((ka, kb)) / math.sqrt(n)
+bi, si = prepare_basis(inp.operation, 2, rec)
+E, V, _, ground = ctx.diagonalization(it, si, bi, E_old, im)
+hop = inp.rescaled_chains()[1][it - inp.indexOfFirstIteration, 0]
+shift = ground - E[int(si[0, 4]) - 1]
+for q in si:
+    d, c0, b0 = int(q[2]), int(q[3]) - 1, int(q[4]) - 1
+    ref, op = bi[b0:b0 + d, 2] - 1, bi[b0:b0 + d, 4]
+    H = np.diag(math.sqrt(inp.Lambda) * E_old[ref])
+    for (a, b, t, _), c in zip(inp.coefficient_diagonalization_type, inp.coefficient_diagonalization):
+        I, J = np.nonzero(op == a)[0], np.nonzero(op == b)[0]
+        B = hop * c * im[np.ix_(ref[J], ref[I], [t - 1])][:, :, 0].T
+        H[np.ix_(I, J)], H[np.ix_(J, I)] = B, B.T
+    h = torch.from_numpy(H).cuda()
+    v = torch.from_numpy(V[c0:c0 + d * d].reshape((d, d), order="F").copy()).cuda()
+    e = torch.from_numpy(E[b0:b0 + d] + shift).cuda()
+    tol = 20 * d * np.finfo(np.float64).eps
+    assert torch.all(torch.diff(e) >= 0)
+    assert (v.T @ v - torch.eye(d, dtype=v.dtype, device="cuda")).abs().max() <= tol
+    assert (h @ v - v * e).abs().max() <= tol * max(1.0, e.abs().max().item())
+    print("order", d)
+"""
+
+
+def test_both_reductions_in_one_group():
+    """Sectors beside the streamed reduction's limit (3536), in one size group: 3600 on the multi-kernel
+    reduction, 3500 streamed.  Residual and orthogonality as in test_gpu_tri_resident, on the device."""
+    root = os.path.dirname(HERE)
+    code = MIXED.format(root=root, package=os.path.join(root, "nrg-mpi_b200"))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, NRG_ENTRY_SOLVER="device"), cwd=root,
+                       capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
+    assert r.stdout.count("order 3600") == 2 and r.stdout.count("order 3500") == 2
