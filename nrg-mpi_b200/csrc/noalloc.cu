@@ -12,6 +12,7 @@ namespace {
 
 // largest block order the static workspace covers
 constexpr long long kMaxN = NRG_NOALLOC_MAX_ORDER;
+constexpr int kPanelOnly = 5;   // see the call
 // [0, 8): sector descriptor, [8, 16): status word and the mark of a close decision, then the
 // workspace
 constexpr long long kDescOff = 0, kStatusOff = 8, kDblOff = 16;
@@ -138,14 +139,20 @@ extern "C" int nrg_block_eigh_noalloc(const double* H, int32_t n, double* eigenv
     NRG_CUDA_TRY(cudaMemcpyAsync(d_sec, &sec, sizeof(sec), cudaMemcpyHostToDevice, st));
     if (eigenvectors != H)
         NRG_CUDA_TRY(cudaMemcpyAsync(eigenvectors, H, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st));
-    // The fast solver, and where it decides so close to a tolerance that a column's sign hangs on
-    // its last bits the panel solver, whose signs stay what they are (eig_panel.cu).  Order 128:
-    // 0.45 ms, 1.9 ms for the 10% that are solved twice; the panel solver alone takes 1.5.
-    double* kept = d_ws + (long long)n * n;   // in place: the block, where only the panel solver works
-    if (eigenvectors == H)
-        NRG_CUDA_TRY(cudaMemcpyAsync(kept, H, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st));
-    NRG_TRY(launch_syev(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, d_status, st));
-    NRG_TRY(launch_syev_panel(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, eigenvectors == H ? kept : H, d_status, st));
+    // Up to order 5 the panel solver alone, one launch instead of three: order 2 takes 51 us for 56,
+    // 3 64 for 61, 4 64 for 68, 5 76 for 81, 6 80..88 for 81, 8 89 for 81.  Above it the fast solver,
+    // and where that decides so close to a tolerance that a column's sign hangs on its last bits the
+    // panel solver, whose signs stay what they are (eig_panel.cu).  Order 128: 0.45 ms, 1.9 ms for
+    // the 10% that are solved twice; the panel solver alone takes 1.5.
+    if (n <= kPanelOnly) {
+        NRG_TRY(launch_syev_panel(d_sec, 1, eigenvectors, eigenvalues, d_ws, nullptr, nullptr, d_status, st));
+    } else {
+        double* kept = d_ws + (long long)n * n;   // in place: the block, where only the panel solver works
+        if (eigenvectors == H)
+            NRG_CUDA_TRY(cudaMemcpyAsync(kept, H, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st));
+        NRG_TRY(launch_syev(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, d_status, st));
+        NRG_TRY(launch_syev_panel(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, eigenvectors == H ? kept : H, d_status, st));
+    }
     int flags = 0;
     NRG_CUDA_TRY(cudaMemcpyAsync(&flags, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     NRG_CUDA_TRY(cudaStreamSynchronize(st));
