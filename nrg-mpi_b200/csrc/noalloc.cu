@@ -147,11 +147,13 @@ extern "C" int nrg_block_eigh_noalloc(const double* H, int32_t n, double* eigenv
     if (n <= kPanelOnly) {
         NRG_TRY(launch_syev_panel(d_sec, 1, eigenvectors, eigenvalues, d_ws, nullptr, nullptr, d_status, st));
     } else {
-        double* kept = d_ws + (long long)n * n;   // in place: the block, where only the panel solver works
-        if (eigenvectors == H)
+        // the block, for the panel solver, where the results are written over it
+        const bool over = eigenvectors == H || (eigenvalues < H + (size_t)n * n && H < eigenvalues + n);
+        double* kept = d_ws + (long long)n * n;   // where only the panel solver works
+        if (over)
             NRG_CUDA_TRY(cudaMemcpyAsync(kept, H, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st));
         NRG_TRY(launch_syev(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, d_status, st));
-        NRG_TRY(launch_syev_panel(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, eigenvectors == H ? kept : H, d_status, st));
+        NRG_TRY(launch_syev_panel(d_sec, 1, eigenvectors, eigenvalues, d_ws, d_unsure, over ? kept : H, d_status, st));
     }
     int flags = 0;
     NRG_CUDA_TRY(cudaMemcpyAsync(&flags, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));

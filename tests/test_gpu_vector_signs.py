@@ -63,3 +63,22 @@ def test_block_signs(n, seed, in_place):
         entry = g[f"entry_{n}_{seed}"]
         negative = np.unpackbits(g[f"negative_{n}_{seed}"], count=n).astype(bool)
     assert np.array_equal(np.nonzero((V[entry, np.arange(n)] < 0) != negative)[0], [])
+
+
+@pytest.mark.parametrize("n,seed,at", [(5, 1, 0), (17, 3, 0), (128, 2456, 0), (128, 2456, 128 * 128 - 128)])
+def test_eigenvalues_over_the_block(n, seed, at):
+    """The eigenvalues may take the block's own storage: the last blocks are solved a second time, from
+    the block as it was given."""
+    rng = np.random.default_rng(10000 + seed)
+    H = rng.standard_normal((n, n)) / math.sqrt(n)
+    H = (H + H.T) / 2 + np.diag(np.sort(7.0 * rng.random(n) ** 0.45))
+    fn = load_library().nrg_block_eigh_noalloc
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    h = torch.from_numpy(H).cuda()
+    E = h.view(-1)[at:at + n]
+    V = torch.zeros_like(h)
+    assert fn(h.data_ptr(), n, E.data_ptr(), V.data_ptr(), None) == 0
+    E, V = E.cpu().numpy(), V.cpu().numpy().T
+    tol = 20 * n * np.finfo(np.float64).eps
+    assert np.max(np.abs(H @ V - V * E)) < tol * np.linalg.norm(H, 2)
+    assert np.max(np.abs(V.T @ V - np.eye(n))) < tol
