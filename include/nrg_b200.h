@@ -272,8 +272,8 @@ NRG_API int nrg_spike_cfs(nrg_context* ctx, int32_t iteration, const nrg_spike_i
  * host application whose pool allocator owns the whole device, or a caller that must not
  * trigger the implicit device synchronisation of cudaMalloc/cudaFree inside a pipelined
  * stream of work.  Diagonalises one symmetric FP64 block (column-major, order n <=
- * NRG_NOALLOC_MAX_ORDER) with the same per-sector eigensolver kernel nrg_diagonalization
- * uses (without the |V| < 1e-14 chop): eigenvalues ascending, eigenvectors in the same
+ * NRG_NOALLOC_MAX_ORDER) with the per-sector eigensolver kernels (without the |V| < 1e-14
+ * chop of nrg_diagonalization): eigenvalues ascending, eigenvectors in the same
  * column order.  H, eigenvalues and eigenvectors are caller-owned device arrays (H may
  * equal eigenvectors).  No context is needed: the call runs on the current device and on
  * `stream` (NULL = default stream), and returns after the stream has drained.
@@ -312,7 +312,7 @@ NRG_API int nrg_host_free(void* p);
  * after the first iteration, the basis records and row lists of prepareBasis
  * (prepareBasis.F90:31-114); the host keeps a few integers per sector.  Models whose
  * operations change the quantum numbers alike (ties in sortBasisArray's exchange sort)
- * build the records on the host, where that exchange sequence is replayed.  Setting the
+ * build the records on the host, in the order that exchange sort leaves.  Setting the
  * environment variable NRG_HOST_TABLES=1 keeps all the bookkeeping on the host;
  * NRG_CHECK_TABLES=1 compares the device's tables with the host's at every iteration and
  * fails the run (NRG_ERR_STATE) on any difference. */

@@ -1,7 +1,9 @@
 // Batched FP64 symmetric eigensolver for the symmetry-sector blocks of one NRG
 // iteration (the dsyev('V','U') call of diagonalization.F90:267, one call per sector),
-// one thread block per sector.  Used for blocks of order <= 128 (large blocks go through
-// the multi-kernel pipeline of eig_large.cu, which reuses the pieces below):
+// one thread block per sector.  Used for blocks of order <= 128 of the runs that keep their
+// eigenvectors on the device, and for nrg_block_eigh_noalloc (large blocks go through
+// the multi-kernel pipeline of eig_large.cu, which reuses the pieces below; the eigenvectors
+// that nrg_diagonalization returns come from eig_panel.cu):
 //   1. Householder tridiagonalisation (H = Q T Q^T) by a launch of its own with the block in
 //      registers (eig_tri.cu), reflectors kept in the block's own storage;
 //   2. divide and conquer on T (eig_dc.cuh: Cuppen tearing down to 1x1 leaves, deflation of

@@ -2,7 +2,7 @@
 // over the whole GPU instead of one block per sector.  All large sectors advance together:
 //   1. Householder tridiagonalisation (eig_tri.cu): orders up to 512 with the matrix on
 //      chip, larger ones streamed from L2 until the trailing block fits there.  Orders
-//      beyond the streaming kernel's shared memory (about 3,600) take the kernels below,
+//      beyond the streaming kernel's shared memory (3,536) take the kernels below,
 //      blocked by panels of 32 columns (the dlatrd scheme): per column one block per sector
 //      updates the column with the pending panel reflectors and forms the Householder
 //      vector, then a many-block kernel computes the symmetric matrix-vector product with

@@ -28,11 +28,12 @@
 // will not wait for it: st.async may still be in flight when its sender has passed a cluster
 // barrier, so only a receiver's wait shows that it is done and the receiver may leave.
 //
-// Against the panel kernel (eig_large.cu), which streams the trailing matrix from L2 and
-// crosses two cluster barriers and about eight block barriers per column: 1.5..2.4 us per
-// column for 6.5..7; order 128 0.20 ms for 0.9 (the one-block code it replaces), 512 1.2 ms
-// for 3.3.  Whole runs: N_keep = 250 37.5 ms for 53, N_keep = 2048 with the FDM spectrum
-// 453 ms for 567, eight models side by side 146 ms for 218.
+// Against the panel kernels (eig_panel.cu), which stream the trailing matrix from L2 and
+// cross two cluster barriers and about eight block barriers per column: 1.5..2.4 us per
+// column for 6.5..7; order 128 0.20 ms for 0.9 (one block there), 512 1.2 ms for 3.3.  With this
+// reduction alone whole runs went to 37.5 ms from 53 (N_keep = 250), 453 from 567 (N_keep =
+// 2048 with the FDM spectrum) and 146 from 218 (eight models side by side); with the divide and
+// conquer of eig_dc.cuh as well they take 21.4, 283 and 102.
 #include "cta_gemm.cuh"
 #include "internal.hpp"
 
@@ -574,8 +575,9 @@ __global__ void __launch_bounds__(kTriThreads, 1) k_tri_res(const TriTask* __res
 // the trailing block back.  Bound by the L2 stream of a block (8 m^2 / CL bytes per step, m the
 // trailing order, at 40 of the 44..48 bytes per cycle that eight warps reach) and, below m
 // of about 600, by the chain of the step.  Order 1225: 9.1 ms to order 512 (9.8 before the
-// aligned columns and the 16 x 8 x 8 MMA on row pairs) and 1.1 ms on chip, against 17.2 ms of the cluster kernel with panels of 32 columns and two cluster
-// barriers per column that it replaced (8 blocks; with 16 that one was no faster).
+// aligned columns and the 16 x 8 x 8 MMA on row pairs) and 1.1 ms on chip, against 17.2 ms of
+// eig_panel.cu's cluster kernel (panels of 32 columns, two cluster barriers per column, 8 blocks;
+// with 16 that one is no faster).
 constexpr int kStreamSlots = 7;   // kept updates at most (NBS), fewer where they do not fit
 
 struct StreamTask {

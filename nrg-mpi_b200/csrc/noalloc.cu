@@ -1,4 +1,4 @@
-// nrg_block_eigh_noalloc: the per-sector FP64 eigensolver of nrg_diagonalization for one
+// nrg_block_eigh_noalloc: the per-sector FP64 eigensolvers (eig.cu, eig_panel.cu) for one
 // symmetric block, for callers that cannot allocate device memory.  Its workspace lives in
 // the file-scope device array below (allocated when the library is loaded on a device and
 // held until the process exits); the call itself allocates nothing.
